@@ -46,14 +46,11 @@ LYM_D cx<double> gen<3>(int a, int i, int j) {
   return {i == 2 ? -2.0 * s3 : s3, 0.0};
 }
 
-// The block's copies of the generators and of the adjoint generators
-// (T_adj^k)_{ij} = -2 Tr([T_k, T_i] T_j) (lie_generators.py:22-36), built once
-// per block in shared memory.
+// The block's copies of the generators, built once per block in shared memory.
 template <int NC>
 struct AdjTables {
   static constexpr int A = NC * NC - 1;
   cx<double> T[A][NC][NC];
-  cx<double> TA[A][A][A];
 };
 
 template <int NC>
@@ -64,35 +61,22 @@ LYM_D void build_tables(AdjTables<NC>& tb) {
     tb.T[a][i][j] = gen<NC>(a, i, j);
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < A * A * A; e += blockDim.x) {
-    const int k = e / (A * A), i = (e / A) % A, j = e % A;
-    // Tr([T_k, T_i] T_j) = sum_{p,q,r} (T_k[p][q] T_i[q][r] - T_i[p][q] T_k[q][r]) T_j[r][p]
-    cx<double> t = czero<double>();
-    for (int p = 0; p < NC; ++p)
-      for (int q = 0; q < NC; ++q)
-        for (int r = 0; r < NC; ++r) {
-          const cx<double> c = tb.T[k][p][q] * tb.T[i][q][r] - tb.T[i][p][q] * tb.T[k][q][r];
-          t += c * tb.T[j][r][p];
-        }
-    tb.TA[k][i][j] = -2.0 * t;
-  }
-  __syncthreads();
 }
 
-// (1 -+ gamma_mu), times gamma_d when hermitian (dirac.py:310-320), element (m, n)
-template <int ND, bool HERM>
-LYM_D cx<double> projector(int mu, double sgn, int m, int n) {
-  constexpr int NS = Gamma<ND>::NS;
-  cx<double> g = czero<double>();
+// U_mu(site), or U_mu(site)^dag when !fwd
+template <int NC>
+LYM_D Mat<NC> load_hop_link(const double2* __restrict__ U, int mu, int64_t site, int64_t V, bool fwd) {
+  Mat<NC> r;
+  const double2* base = U + (int64_t)mu * NC * NC * V + site;
+  const double s = fwd ? 1.0 : -1.0;
 #pragma unroll
-  for (int a = 0; a < NS / 2; ++a) {
-    const int jb = Gamma<ND>::col(mu, a), ph = Gamma<ND>::phase(mu, a);
-    if (m == a && n == jb) g = mul_phase(ph, cx<double>{1.0, 0.0});
-    if (m == jb && n == a) g = mul_phase(phase_conj(ph), cx<double>{1.0, 0.0});
-  }
-  cx<double> p = {(m == n ? 1.0 : 0.0) - sgn * g.re, -sgn * g.im};
-  if (HERM && m >= NS / 2) p = -p;
-  return p;
+  for (int i = 0; i < NC; ++i)
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      const cx<double> t = ld(base + (fwd ? i * NC + j : j * NC + i) * V);
+      r.m[i][j] = {t.re, s * t.im};
+    }
+  return r;
 }
 
 LYM_D size_t adj_index(int s, int i, int j, int NC, int64_t V, int64_t x) {
@@ -102,89 +86,104 @@ LYM_D size_t adj_index(int s, int i, int j, int NC, int64_t V, int64_t x) {
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// operator: one thread per (site, colour row i, vector)
+// operator: one thread per (site, upper spin row a, vector); in 4D the two threads of
+// a site are lanes l and l + 16 of one warp (16 consecutive sites per warp).
+//
+// Row a of the upper half spinor h = psi_a - s g_a psi_ja feeds the output rows a and
+// j_a, where j_a is 3 - a (mu = 0, 1) or 2 + a (mu = 2, 3): after mu = 1 the two threads
+// swap their lower rows, which makes the partner's 3 - (1 - a) this thread's 2 + a, so
+// two rows are live at a time.  No spinor value is loaded by both threads; the link is,
+// from the same addresses of the same instruction.  (A thread per colour row loaded the
+// whole neighbour spinor N times.)  Latency-bound at 8 warps per SM (255 registers);
+// 16^4 SU(3): 47 us against 75 us, the FP64 work alone is 13 us.  Three or four blocks per
+// SM spill and take 59 and 87 us; a real loop over the directions 54 to 62 us.
+// LR: the left links are another field than the right ones.
 // ---------------------------------------------------------------------------
-template <int ND, int NC, bool HERM>
-__global__ void __launch_bounds__(kAdjBlock, 1) wilson_adjoint_kernel(
+template <int ND, int NC, bool HERM, bool LR>
+__global__ void __launch_bounds__(kAdjBlock, 2) wilson_adjoint_kernel(
     const int32_t* __restrict__ tab, int V, int Lt, double kappa, double bcr, double bci,
     const double2* __restrict__ UL, const double2* __restrict__ UR, const double2* __restrict__ in,
     double2* __restrict__ out) {
-  constexpr int NS = Gamma<ND>::NS;
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int i = blockIdx.y;
-  if (x >= V) return;
+  constexpr int NS = Gamma<ND>::NS, NA = NS / 2;  // NA threads per site
+  constexpr int SW = 32 / NA;                     // sites per warp
+  const int lane = threadIdx.x & 31;
+  const int a = NA == 2 ? lane >> 4 : 0;
+  const int xs = (int)(blockIdx.x * (kAdjBlock / 32) + (threadIdx.x >> 5)) * SW + (lane % SW);
+  const int x = xs < V ? xs : V - 1;  // every lane takes part in the exchange below
   const size_t vec = (size_t)NS * NC * NC * V;
-  const double2* psi = in + blockIdx.z * vec;
-  double2* res = out + blockIdx.z * vec;
+  const double2* psi = in + blockIdx.y * vec;
+  double2* res = out + blockIdx.y * vec;
   const cx<double> bc{bcr, bci};
-  cx<double> acc[NS][NC];
-#pragma unroll
-  for (int s = 0; s < NS; ++s)
-#pragma unroll
-    for (int l = 0; l < NC; ++l) acc[s][l] = czero<double>();
+  Mat<NC> up = mzero<NC>(), low = mzero<NC>();
 
+  // forward M = U(x), backward M = U(x - mu)^dag, both o = M h M^dag
 #pragma unroll
-  for (int mu = 0; mu < ND; ++mu) {
+  for (int md = 0; md < 2 * ND; ++md) {
+    const int mu = md >> 1;
+    const bool fwd = (md & 1) == 0;
+    if (NA == 2 && md == 4) {
 #pragma unroll
-    for (int dir = 0; dir < 2; ++dir) {
-      const bool fwd = dir == 0;
-      const int y = tab[(fwd ? 0 : ND) * V + mu * V + x];
-      const int site = fwd ? x : y;  // the link's site: x forward, x - mu backward
-      const bool boundary = mu == ND - 1 && (fwd ? (x % Lt) == Lt - 1 : (x % Lt) == 0);
-      // left factor: row i of L (forward) or of L^dag (backward); right factor R in full
-      cx<double> lrow[NC];
-#pragma unroll
-      for (int j = 0; j < NC; ++j) {
-        cx<double> v = fwd ? ld(UL + ((size_t)(mu * NC + i) * NC + j) * V + site)
-                           : conj(ld(UL + ((size_t)(mu * NC + j) * NC + i) * V + site));
-        if (boundary) v = fwd ? bc * v : conj(bc) * v;
-        lrow[j] = v;
-      }
-      cx<double> r[NC][NC];
-#pragma unroll
-      for (int p = 0; p < NC; ++p)
-#pragma unroll
-        for (int q = 0; q < NC; ++q) r[p][q] = ld(UR + ((size_t)(mu * NC + p) * NC + q) * V + site);
-      const double sgn = fwd ? 1.0 : -1.0;
-#pragma unroll
-      for (int a = 0; a < NS / 2; ++a) {
-        const int jb = Gamma<ND>::col(mu, a), ph = Gamma<ND>::phase(mu, a);
-        // w = lrow . h with h = psi_a - s g_a psi_jb (N x N); then o = w R^dag (forward) or w R
-        cx<double> w[NC];
-#pragma unroll
-        for (int l = 0; l < NC; ++l) w[l] = czero<double>();
-#pragma unroll
-        for (int j = 0; j < NC; ++j)
-#pragma unroll
-          for (int l = 0; l < NC; ++l) {
-            const cx<double> h = ld(psi + adj_index(a, j, l, NC, V, y)) -
-                                 sgn * mul_phase(ph, ld(psi + adj_index(jb, j, l, NC, V, y)));
-            cmac(w[l], lrow[j], h);
-          }
-        const int lph = fwd ? phase_neg(phase_conj(ph)) : phase_conj(ph);
+      for (int i = 0; i < NC; ++i)
 #pragma unroll
         for (int l = 0; l < NC; ++l) {
-          cx<double> o = czero<double>();
-#pragma unroll
-          for (int q = 0; q < NC; ++q) {
-            if (fwd) cmac(o, w[q], conj(r[l][q]));  // (w R^dag)_l = sum_q w_q conj(R[l][q])
-            else cmac(o, w[q], r[q][l]);            // (w R)_l
-          }
-          acc[a][l] += o;
-          acc[jb][l] += mul_phase(lph, o);
+          low.m[i][l].re = __shfl_xor_sync(0xffffffffu, low.m[i][l].re, 16);
+          low.m[i][l].im = __shfl_xor_sync(0xffffffffu, low.m[i][l].im, 16);
         }
+    }
+    const int y = tab[(fwd ? 0 : ND) * V + mu * V + x];
+    const int site = fwd ? x : y;  // the link's site: x forward, x - mu backward
+    const bool boundary = mu == ND - 1 && (fwd ? (x % Lt) == Lt - 1 : (x % Lt) == 0);
+    const double sg = fwd ? 1.0 : -1.0;
+    const bool im = gamma_imag<ND>(mu);
+    const double g = gamma_sign<ND>(mu, a);
+    Mat<NC> h;
+    {
+      const double2* pu = psi + adj_index(a, 0, 0, NC, V, y);
+      const double2* pl = psi + adj_index(Gamma<ND>::col(mu, a), 0, 0, NC, V, y);
+#pragma unroll
+      for (int k = 0; k < NC * NC; ++k) {
+        cx<double> t = ld(pu + (size_t)k * V);
+        add_gamma(t, -sg * g, im, ld(pl + (size_t)k * V));
+        h.m[k / NC][k % NC] = t;
+      }
+    }
+    const Mat<NC> r = load_hop_link<NC>(UR, mu, site, V, fwd);
+    Mat<NC> ll;
+    if constexpr (LR) ll = load_hop_link<NC>(UL, mu, site, V, fwd);
+    else ll = r;
+#pragma unroll
+    for (int i = 0; i < NC; ++i) {
+      cx<double> w[NC];
+      row_mul<NC>(w, ll.m[i], h);
+      if (boundary) {
+#pragma unroll
+        for (int l = 0; l < NC; ++l) w[l] = (fwd ? bc : conj(bc)) * w[l];
+      }
+      cx<double> o[NC];
+#pragma unroll
+      for (int l = 0; l < NC; ++l) o[l] = czero<double>();
+      row_mac_nd<NC>(o, w, r);
+#pragma unroll
+      for (int l = 0; l < NC; ++l) {
+        up.m[i][l] += o[l];
+        add_gamma(low.m[i][l], im ? sg * g : -sg * g, im, o[l]);  // -s conj(g) o
       }
     }
   }
+  if (xs >= V) return;
 #pragma unroll
-  for (int s = 0; s < NS; ++s)
+  for (int half = 0; half < 2; ++half) {
+    const Mat<NC>& acc = half ? low : up;
 #pragma unroll
-    for (int l = 0; l < NC; ++l) {
-      const size_t k = adj_index(s, i, l, NC, V, x);
-      cx<double> v = ld(psi + k) + kappa * acc[s][l];
-      if (HERM && s >= NS / 2) v = -v;
-      st(res + k, v);
-    }
+    for (int i = 0; i < NC; ++i)
+#pragma unroll
+      for (int l = 0; l < NC; ++l) {
+        const size_t k = adj_index(half * (NS / 2) + a, i, l, NC, V, x);
+        cx<double> v = ld(psi + k) + kappa * acc.m[i][l];
+        if (HERM && half) v = -v;
+        st(res + k, v);
+      }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -223,107 +222,125 @@ __global__ void __launch_bounds__(kAdjBlock) adjoint_links_kernel(int nd, int64_
 
 // ---------------------------------------------------------------------------
 // fermion force: one thread per (site, mu)
+//
+// The reference contracts adjoint components (dirac.py:547-560):
+//   c_k = sum_ij TA^k_ij sum_m [conj(X_m)_i (P+ Z)_mj - conj(Z_m)_i (P- X)_mj],  Z = V Y(x + mu)
+// with TA^k_ij = -2 Tr([T_k, T_i] T_j), and the force is sum_k c_k T_k.  In matrices,
+// Z = U Y U^dag, and by the completeness of the T_k (2 sum_k T_k Tr(T_k C) = C for
+// traceless C) the whole contraction is
+//   sum_k c_k T_k = -sum_m ([X_m^dag, (P+ Z)_m] - [Z_m^dag, (P- X)_m])
+// (the trace parts of X and Z drop out of the commutators; Y's is removed first).
+// The projectors have rank two: with h+- = X_a +- g_a X_ja and z+- = U (Y_a +- g_a Y_ja) U^dag
+// over the upper rows a,
+//   gamma_d (1 -+ gamma):  -sum_a (K_a - K_a^dag),  K_a = h+^dag z-  - z- h+^dag
+//   (1 -+ gamma):          -sum_a ([h-^dag, z-] - [z+^dag, h+])
+// so a pole costs 16 (hermitian) N x N products per link instead of the (N^2-1)-component
+// contraction through local memory (the neighbour loads now bound it): 8^3 x 16 SU(3), 4 poles: 34 us against 870 us.
 // ---------------------------------------------------------------------------
 constexpr int kMaxAdjForceTerms = 32;
 struct AdjForceTerms {
   double alpha[kMaxAdjForceTerms];
 };
 
-// c_k += w * sum_ij TA[k][i][j] M_ij for L(P, Q) at this link, M_ij =
-// sum_m [conj(Pv_m)_i (P+ Z)_{m j} - conj(Z_m)_i (P- Pv)_{m j}], Z_n = V Qv_n
-// (the two einsums of dirac.py:547-560 with the adjoint components).
-template <int ND, int NC, bool HERM>
-LYM_D void adjoint_lie_term(const AdjTables<NC>& tb, int mu, const cx<double> (&Vm)[NC * NC - 1][NC * NC - 1],
-                            const cx<double> (&Pv)[Gamma<ND>::NS][NC * NC - 1],
-                            const cx<double> (&Qv)[Gamma<ND>::NS][NC * NC - 1], double w, cx<double> (&c)[NC * NC - 1]) {
-  constexpr int NS = Gamma<ND>::NS, A = NC * NC - 1;
-  cx<double> Z[NS][A], PZ[NS][A], PP[NS][A];
-  for (int n = 0; n < NS; ++n)
-    for (int a = 0; a < A; ++a) {
-      cx<double> t = czero<double>();
-      for (int b = 0; b < A; ++b) t += Vm[a][b] * Qv[n][b];
-      Z[n][a] = t;
-    }
-  for (int m = 0; m < NS; ++m)
-    for (int a = 0; a < A; ++a) {
-      cx<double> zp = czero<double>(), pm = czero<double>();
-      for (int n = 0; n < NS; ++n) {
-        zp += projector<ND, HERM>(mu, 1.0, m, n) * Z[n][a];
-        pm += projector<ND, HERM>(mu, -1.0, m, n) * Pv[n][a];
+// psi_a + s g_a psi_ja at site x
+template <int ND, int NC>
+LYM_D Mat<NC> adj_half(const double2* __restrict__ f, int mu, int a, bool plus, int64_t V, int64_t x) {
+  const bool im = gamma_imag<ND>(mu);
+  const double g = plus ? gamma_sign<ND>(mu, a) : -gamma_sign<ND>(mu, a);
+  const double2* pu = f + adj_index(a, 0, 0, NC, V, x);
+  const double2* pl = f + adj_index(Gamma<ND>::col(mu, a), 0, 0, NC, V, x);
+  Mat<NC> h;
+#pragma unroll
+  for (int k = 0; k < NC * NC; ++k) {
+    cx<double> t = ld(pu + k * V);
+    add_gamma(t, g, im, ld(pl + k * V));
+    h.m[k / NC][k % NC] = t;
+  }
+  return h;
+}
+
+template <int NC>
+LYM_D void remove_trace(Mat<NC>& m) {
+  const cx<double> t = (1.0 / NC) * trace(m);
+#pragma unroll
+  for (int i = 0; i < NC; ++i) m.m[i][i] -= t;
+}
+
+// K += w [h^dag, z]
+template <int NC>
+LYM_D void commutator_mac(Mat<NC>& K, double w, const Mat<NC>& h, const Mat<NC>& z) {
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      cx<double> t = cmul_cj(h.m[0][i], z.m[0][j]);
+#pragma unroll
+      for (int k = 1; k < NC; ++k) cmac_cj(t, h.m[k][i], z.m[k][j]);
+#pragma unroll
+      for (int k = 0; k < NC; ++k) {  // - z_ik conj(h_jk)
+        const cx<double> n = -z.m[i][k];
+        cmac_cj(t, h.m[j][k], n);
       }
-      PZ[m][a] = zp;
-      PP[m][a] = pm;
-    }
-  for (int i = 0; i < A; ++i)
-    for (int j = 0; j < A; ++j) {
-      cx<double> mij = czero<double>();
-      for (int m = 0; m < NS; ++m) mij += cmul_cj(Pv[m][i], PZ[m][j]) - cmul_cj(Z[m][i], PP[m][j]);
-      for (int k = 0; k < A; ++k) c[k] += w * (tb.TA[k][i][j] * mij);
+      K.m[i][j] += w * t;
     }
 }
 
+// In 4D the two upper rows of a link are two threads, lanes l and l + 16 of a warp (16
+// sites), added by a shuffle at the end: the poles of a link are a serial chain of loads,
+// and the small lattices of this force leave the chip half empty with a thread per link.
 template <int ND, int NC, bool HERM>
-__global__ void __launch_bounds__(kAdjBlock) adjoint_force_kernel(
+__global__ void __launch_bounds__(kAdjBlock, 2) adjoint_force_kernel(
     const int32_t* __restrict__ tab, int64_t V, int Lt, double kappa, double bcr, double bci,
     const double2* __restrict__ U, int nterms, AdjForceTerms terms, const double2* __restrict__ X,
     const double2* __restrict__ Y, int symmetric, double scale, double2* __restrict__ force) {
-  constexpr int NS = Gamma<ND>::NS, A = NC * NC - 1;
-  __shared__ AdjTables<NC> tb;
-  build_tables<NC>(tb);
-  const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int mu = blockIdx.y;
-  if (x >= V) return;
+  constexpr int NS = Gamma<ND>::NS, NA = NS / 2, SW = 32 / NA;
+  const int lane = threadIdx.x & 31, a = NA == 2 ? lane >> 4 : 0;
+  const int64_t wid = (int64_t)blockIdx.x * (kAdjBlock / 32) + (threadIdx.x >> 5), sb = wid / ND;
+  const int mu = (int)(wid - sb * ND);  // the directions of a site block run side by side
+  const int64_t xs = sb * SW + lane % SW;
+  const int64_t x = xs < V ? xs : V - 1;  // every lane takes part in the shuffle
   const int64_t y = tab[mu * V + x];
-  // adjoint link of this link, boundary factor on the last time slice
-  Mat<NC> u = load_link<NC>(U, mu, x, V);
+  const Mat<NC> u = load_link<NC>(U, mu, x, V);
   const bool boundary = mu == ND - 1 && (x % Lt) == Lt - 1;
   const cx<double> f = boundary ? cx<double>{bcr, bci} : cx<double>{1.0, 0.0};
-  cx<double> Vm[A][A];
-  for (int b = 0; b < A; ++b) {
-    Mat<NC> tbm;
-    for (int p = 0; p < NC; ++p)
-      for (int q = 0; q < NC; ++q) tbm.m[p][q] = tb.T[b][p][q];
-    const Mat<NC> w = mul_nd(mul(u, tbm), u);
-    for (int a = 0; a < A; ++a) {
-      cx<double> t = czero<double>();
-      for (int p = 0; p < NC; ++p)
-        for (int q = 0; q < NC; ++q) t += tb.T[a][p][q] * w.m[q][p];
-      Vm[a][b] = f * (2.0 * t);
-    }
-  }
-  cx<double> c[A];
-  for (int k = 0; k < A; ++k) c[k] = czero<double>();
+  Mat<NC> K = mzero<NC>();
   const size_t vec = (size_t)NS * NC * NC * V;
   for (int term = 0; term < nterms; ++term) {
-    const double2* Xk = X + term * vec;
-    const double2* Yk = Y + term * vec;
-    // adjoint components 2 Tr(T_a M) of X, Y at x and at x + mu
-    cx<double> xv[NS][A], yv[NS][A];
+    const double w = kappa * terms.alpha[term];
     for (int side = 0; side < (symmetric ? 2 : 1); ++side) {
-      const double2* P = side == 0 ? Xk : Yk;  // L(P, Q): P at x, Q at x + mu
-      const double2* Q = side == 0 ? Yk : Xk;
-      for (int s = 0; s < NS; ++s)
-        for (int a = 0; a < A; ++a) {
-          cx<double> tp = czero<double>(), tq = czero<double>();
-          for (int p = 0; p < NC; ++p)
-            for (int q = 0; q < NC; ++q) {
-              tp += tb.T[a][p][q] * ld(P + adj_index(s, q, p, NC, V, x));
-              tq += tb.T[a][p][q] * ld(Q + adj_index(s, q, p, NC, V, y));
-            }
-          xv[s][a] = 2.0 * tp;
-          yv[s][a] = 2.0 * tq;
-        }
-      adjoint_lie_term<ND, NC, HERM>(tb, mu, Vm, xv, yv, kappa * terms.alpha[term], c);
+      const double2* P = (side == 0 ? X : Y) + term * vec;  // L(P, Q): P at x, Q at x + mu
+      const double2* Q = (side == 0 ? Y : X) + term * vec;
+#pragma unroll 1
+      for (int c = 0; c < (HERM ? 1 : 2); ++c) {
+        const bool plus = c == 1;  // the second commutator of the plain projector
+        Mat<NC> q = adj_half<ND, NC>(Q, mu, a, plus, V, y);
+        remove_trace<NC>(q);  // the components have no trace part, whatever U is
+        const Mat<NC> h = adj_half<ND, NC>(P, mu, a, HERM || plus, V, x);
+        Mat<NC> z = mul_nd(mul(u, q), u);
+        if (boundary) z = mscale(f, z);
+        if (HERM || !plus) commutator_mac<NC>(K, w, h, z);
+        else commutator_mac<NC>(K, -w, z, h);
+      }
     }
   }
-  Mat<NC> out = load_link<NC>(force, mu, x, V);
+  if constexpr (NA == 2) {
+#pragma unroll
+    for (int p = 0; p < NC; ++p)
+#pragma unroll
+      for (int q = 0; q < NC; ++q) {
+        K.m[p][q].re += __shfl_xor_sync(0xffffffffu, K.m[p][q].re, 16);
+        K.m[p][q].im += __shfl_xor_sync(0xffffffffu, K.m[p][q].im, 16);
+      }
+  }
+  if (xs >= V || a != 0) return;
+#pragma unroll
   for (int p = 0; p < NC; ++p)
+#pragma unroll
     for (int q = 0; q < NC; ++q) {
-      cx<double> t = czero<double>();
-      for (int k = 0; k < A; ++k) t += c[k] * tb.T[k][p][q];
-      out.m[p][q] += scale * t;
+      const cx<double> t = HERM ? conj(K.m[q][p]) - K.m[p][q] : -K.m[p][q];
+      double2* o = force + ((int64_t)(mu * NC + p) * NC + q) * V + x;
+      st(o, ld(o) + scale * t);
     }
-  store_link<NC>(force, mu, x, V, out);
 }
 
 }  // namespace lym
@@ -343,18 +360,30 @@ int lym_wilson_apply_adjoint(const lym_lattice* lat, int nc, double kappa, int h
     return LYM_ERR_UNSUPPORTED;
   }
   LYM_REQUIRE(nc == 2 || nc == 3, LYM_ERR_UNSUPPORTED, "N=%d not supported (2 or 3)", nc);
-  dim3 grid(grid_for(lat->V, kAdjBlock), nc, nvec);
+  const int per_block = lat->nd == 4 ? kAdjBlock / 2 : kAdjBlock;  // sites
+  dim3 grid(grid_for(lat->V, per_block), nvec);
   cudaStream_t st = (cudaStream_t)stream;
   const int Lt = lat->dims[lat->nd - 1];
-#define LYM_ADJ(ND_, NC_, H_)                                                                              \
-  wilson_adjoint_kernel<ND_, NC_, H_><<<grid, kAdjBlock, 0, st>>>(lat->d_tab, (int)lat->V, Lt, kappa, bc_re, \
-                                                                  bc_im, (const double2*)gauge_left,       \
-                                                                  (const double2*)gauge, (const double2*)in, \
-                                                                  (double2*)out)
-  if (lat->nd == 2 && nc == 2) { if (hermitian) LYM_ADJ(2, 2, true); else LYM_ADJ(2, 2, false); }
-  else if (lat->nd == 2 && nc == 3) { if (hermitian) LYM_ADJ(2, 3, true); else LYM_ADJ(2, 3, false); }
-  else if (lat->nd == 4 && nc == 2) { if (hermitian) LYM_ADJ(4, 2, true); else LYM_ADJ(4, 2, false); }
-  else { if (hermitian) LYM_ADJ(4, 3, true); else LYM_ADJ(4, 3, false); }
+  const bool lr = gauge_left != gauge;
+#define LYM_ADJ(ND_, NC_, H_, LR_)                                                                         \
+  wilson_adjoint_kernel<ND_, NC_, H_, LR_><<<grid, kAdjBlock, 0, st>>>(                                    \
+      lat->d_tab, (int)lat->V, Lt, kappa, bc_re, bc_im, (const double2*)gauge_left, (const double2*)gauge, \
+      (const double2*)in, (double2*)out)
+#define LYM_ADJ_H(ND_, NC_)                                              \
+  do {                                                                   \
+    if (hermitian) {                                                     \
+      if (lr) LYM_ADJ(ND_, NC_, true, true);                             \
+      else LYM_ADJ(ND_, NC_, true, false);                               \
+    } else {                                                             \
+      if (lr) LYM_ADJ(ND_, NC_, false, true);                            \
+      else LYM_ADJ(ND_, NC_, false, false);                              \
+    }                                                                    \
+  } while (0)
+  if (lat->nd == 2 && nc == 2) LYM_ADJ_H(2, 2);
+  else if (lat->nd == 2 && nc == 3) LYM_ADJ_H(2, 3);
+  else if (lat->nd == 4 && nc == 2) LYM_ADJ_H(4, 2);
+  else LYM_ADJ_H(4, 3);
+#undef LYM_ADJ_H
 #undef LYM_ADJ
   LYM_CHECK_LAUNCH();
   return LYM_OK;
@@ -390,7 +419,8 @@ int lym_fermion_force_adjoint(const lym_lattice* lat, int nc, double kappa, int 
   LYM_REQUIRE(nc == 2 || nc == 3, LYM_ERR_UNSUPPORTED, "N=%d not supported (2 or 3)", nc);
   AdjForceTerms t;
   for (int i = 0; i < kMaxAdjForceTerms; ++i) t.alpha[i] = i < nterms ? alphas[i] : 0.0;
-  dim3 grid(grid_for(lat->V, kAdjBlock), lat->nd);
+  const int sites = lat->nd == 4 ? 16 : 32;  // per warp and direction
+  const unsigned grid = grid_for((lat->V + sites - 1) / sites * lat->nd, kAdjBlock / 32);
   cudaStream_t st = (cudaStream_t)stream;
   const int Lt = lat->dims[lat->nd - 1];
 #define LYM_AF(ND_, NC_, H_)                                                                            \

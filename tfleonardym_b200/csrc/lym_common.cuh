@@ -125,6 +125,25 @@ template <> struct Gamma<3> {
   LYM_HD static int phase(int mu, int) { return mu == 0 ? 0 : 3; }
 };
 
+// g_a of gamma_mu as a real sign and "imaginary" flag (g = s or s i); which of the two it
+// is depends on mu only (2 and 4 dimensions), so kernels that give a row to each thread
+// need no per-thread selection.
+template <int ND> LYM_HD bool gamma_imag(int mu) { return ND == 4 ? (mu & 1) == 0 && mu != 3 : mu == 1; }
+template <int ND> LYM_HD double gamma_sign(int mu, int a) {
+  const int ph = Gamma<ND>::phase(mu, a);  // 0: +1, 1: +i, 2: -1, 3: -i
+  return ph < 2 ? 1.0 : -1.0;
+}
+// t += w g p for the row with g = s (imag = false) or s i; w real
+template <typename T> LYM_HD void add_gamma(cx<T>& t, T ws, bool imag, cx<T> p) {
+  if (imag) {
+    t.re = fma(-ws, p.im, t.re);
+    t.im = fma(ws, p.re, t.im);
+  } else {
+    t.re = fma(ws, p.re, t.re);
+    t.im = fma(ws, p.im, t.im);
+  }
+}
+
 template <typename R, int NC>
 LYM_HD void proj3(int mu, int s, const cx<R> (&p0)[NC], const cx<R> (&p1)[NC], cx<R> (&h)[NC]) {
 #pragma unroll

@@ -47,6 +47,20 @@ LYM_D Mat<N> mident() {
   return r;
 }
 
+// Thread -> link for the kernels that read neighbouring links: warp w of the grid takes
+// direction w mod nd of the 32 sites of site block w / nd, so the directions of a site run
+// side by side in one block and the links they share (44 distinct links per site in 4D
+// against 76 loads) meet in L1; with the direction as the slow grid index every direction
+// streamed the field through L2 on its own.
+LYM_D bool warp_link(int nd, int64_t V, int64_t block, int& mu, int64_t& s) {
+  const int64_t w = block * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int64_t sb = w / nd;
+  mu = (int)(w - sb * nd);
+  s = sb * 32 + (threadIdx.x & 31);
+  return s < V;
+}
+inline unsigned warp_link_grid(int nd, int64_t V, int block) { return grid_for((V + 31) / 32 * nd, block / 32); }
+
 // A B
 template <int N>
 LYM_D Mat<N> mul(const Mat<N>& a, const Mat<N>& b) {
@@ -71,12 +85,39 @@ LYM_D Mat<N> mul_nd(const Mat<N>& a, const Mat<N>& b) {
   for (int i = 0; i < N; ++i)
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      cx<double> t = czero<double>();
+      cx<double> t = cmul_cj(b.m[j][0], a.m[i][0]);
 #pragma unroll
-      for (int k = 0; k < N; ++k) t += a.m[i][k] * conj(b.m[j][k]);
+      for (int k = 1; k < N; ++k) cmac_cj(t, b.m[j][k], a.m[i][k]);
       r.m[i][j] = t;
     }
   return r;
+}
+
+// r = a B for a row vector a
+template <int N>
+LYM_D void row_mul(cx<double> (&r)[N], const cx<double> (&a)[N], const Mat<N>& b) {
+#pragma unroll
+  for (int j = 0; j < N; ++j) {
+    r[j] = a[0] * b.m[0][j];
+#pragma unroll
+    for (int k = 1; k < N; ++k) cmac(r[j], a[k], b.m[k][j]);
+  }
+}
+// s += a B
+template <int N>
+LYM_D void row_mac(cx<double> (&s)[N], const cx<double> (&a)[N], const Mat<N>& b) {
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+#pragma unroll
+    for (int k = 0; k < N; ++k) cmac(s[j], a[k], b.m[k][j]);
+}
+// s += a B^dag
+template <int N>
+LYM_D void row_mac_nd(cx<double> (&s)[N], const cx<double> (&a)[N], const Mat<N>& b) {
+#pragma unroll
+  for (int j = 0; j < N; ++j)
+#pragma unroll
+    for (int k = 0; k < N; ++k) cmac_cj(s[j], b.m[j][k], a[k]);
 }
 
 // A^dag B
@@ -87,9 +128,9 @@ LYM_D Mat<N> mul_dn(const Mat<N>& a, const Mat<N>& b) {
   for (int i = 0; i < N; ++i)
 #pragma unroll
     for (int j = 0; j < N; ++j) {
-      cx<double> t = czero<double>();
+      cx<double> t = cmul_cj(a.m[0][i], b.m[0][j]);
 #pragma unroll
-      for (int k = 0; k < N; ++k) t += cmul_cj(a.m[k][i], b.m[k][j]);
+      for (int k = 1; k < N; ++k) cmac_cj(t, a.m[k][i], b.m[k][j]);
       r.m[i][j] = t;
     }
   return r;
