@@ -408,112 +408,96 @@ __global__ void __launch_bounds__(128) unitary_projection_kernel(int64_t nlinks,
 //   L(X, Y)_{ut} = kappa/2 [A_{tu} - B_{tu} - delta_{ut} (Tr A - Tr B)/N]
 // which is the reference's sum over generators T^k_{ij} T^k_{ut} written with
 // the SU(N) completeness relation sum_k T^k_ij T^k_ut = (d_it d_ju - d_ij d_ut/N)/2.
-// P+- = (1 -+ gamma_mu), multiplied by gamma_d when hermitian.
+// P+- = (1 -+ gamma_mu), multiplied by gamma_d when hermitian.  The projectors have rank
+// ns/2: over the upper rows a, with x+- = X_a +- g_a X_ja and v+- = U (Y_a +- g_a Y_ja)(x+mu),
+//   hermitian:  A = sum_a conj(x+) (x) v-,   B = A^dag (one outer product per row)
+//   plain:      A = sum_a conj(x-) (x) v-,   B = sum_a conj(v+) (x) x+
+// so a link and pole costs ns/2 matvecs and outer products per ordering instead of ns
+// matvecs, two full projections and 2 ns outer products, which spilled; the poles'
+// weights go into the sum.  12^3 x 24 SU(3), 8 poles: 97 us against 336 us, 16^4, 10 poles: 172 us
+// against 620 us (three blocks per SM; two take 180, four spill and take 186); bound by
+// the four spinor gathers per link and pole.
 // ---------------------------------------------------------------------------
 constexpr int kMaxForceTerms = 64;
 struct ForceTerms {
   double alpha[kMaxForceTerms];
 };
 
-// (1 - s gamma_mu) v, optionally times gamma_d, for the reference basis
-template <int ND, int NC, bool HERM>
-LYM_D void project_full(int mu, double sgn, const cx<double> (&v)[Gamma<ND>::NS][NC],
-                        cx<double> (&o)[Gamma<ND>::NS][NC]) {
-  constexpr int NS = Gamma<ND>::NS;
+// one upper row of psi_a + s g_a psi_ja at site x
+template <int ND, int NC>
+LYM_D void half_row(const double2* __restrict__ f, int mu, int a, bool plus, int64_t V, int64_t x,
+                    cx<double> (&h)[NC]) {
+  const bool im = gamma_imag<ND>(mu);
+  const double g = plus ? gamma_sign<ND>(mu, a) : -gamma_sign<ND>(mu, a);
+  const double2* pu = f + (int64_t)a * NC * V + x;
+  const double2* pl = f + (int64_t)Gamma<ND>::col(mu, a) * NC * V + x;
 #pragma unroll
-  for (int a = 0; a < NS / 2; ++a) {
-    const int jb = Gamma<ND>::col(mu, a), ph = Gamma<ND>::phase(mu, a);
-#pragma unroll
-    for (int c = 0; c < NC; ++c) {
-      cx<double> up = v[a][c] - sgn * mul_phase(ph, v[jb][c]);
-      cx<double> lo = v[jb][c] - sgn * mul_phase(phase_conj(ph), v[a][c]);
-      o[a][c] = up;
-      o[jb][c] = HERM ? -lo : lo;
-    }
+  for (int c = 0; c < NC; ++c) {
+    h[c] = ld(pu + c * V);
+    add_gamma(h[c], g, im, ld(pl + c * V));
   }
 }
 
 template <int ND, int NC, bool HERM>
-LYM_D void lie_term(int mu, const Mat<NC>& U, const cx<double> (&X)[Gamma<ND>::NS][NC],
-                    const cx<double> (&Ysup)[Gamma<ND>::NS][NC], Mat<NC>& A, Mat<NC>& B) {
-  constexpr int NS = Gamma<ND>::NS;
-  cx<double> Vv[NS][NC], PV[NS][NC], PX[NS][NC];
-#pragma unroll
-  for (int m = 0; m < NS; ++m)
-#pragma unroll
-    for (int i = 0; i < NC; ++i) {
-      cx<double> t = czero<double>();
-#pragma unroll
-      for (int l = 0; l < NC; ++l) t += U.m[i][l] * Ysup[m][l];
-      Vv[m][i] = t;
-    }
-  project_full<ND, NC, HERM>(mu, 1.0, Vv, PV);
-  project_full<ND, NC, HERM>(mu, -1.0, X, PX);
-#pragma unroll
-  for (int m = 0; m < NS; ++m)
-#pragma unroll
-    for (int i = 0; i < NC; ++i)
-#pragma unroll
-      for (int j = 0; j < NC; ++j) {
-        A.m[i][j] += cmul_cj(X[m][i], PV[m][j]);
-        B.m[i][j] += cmul_cj(Vv[m][i], PX[m][j]);
-      }
-}
-
-template <int ND, int NC, bool HERM>
-__global__ void __launch_bounds__(128) fermion_force_kernel(
+__global__ void __launch_bounds__(128, 3) fermion_force_kernel(
     const int32_t* __restrict__ tab, int64_t V, int Lt, double kappa, double bcr, double bci,
     const double2* __restrict__ U, int nterms, ForceTerms terms, const double2* __restrict__ X,
     const double2* __restrict__ Y, int symmetric, double scale, double2* __restrict__ force) {
   constexpr int NS = Gamma<ND>::NS;
-  const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int mu = blockIdx.y;
-  if (s >= V) return;
+  int mu;
+  int64_t s;
+  if (!warp_link(ND, V, blockIdx.x, mu, s)) return;
   const int64_t y = tab[mu * V + s];
   Mat<NC> u = load_link<NC>(U, mu, s, V);
   if (mu == ND - 1 && (s % Lt) == Lt - 1) u = mscale(cx<double>{bcr, bci}, u);
-  Mat<NC> F = mzero<NC>();
+  Mat<NC> K = mzero<NC>();  // sum over the poles of w (A - B), hermitian: of w A
   const int64_t vec = (int64_t)NS * NC * V;
   for (int k = 0; k < nterms; ++k) {
-    const double2* Xk = X + k * vec;
-    const double2* Yk = Y + k * vec;
-    cx<double> xs[NS][NC], ysup[NS][NC];
-#pragma unroll
-    for (int m = 0; m < NS; ++m)
-#pragma unroll
-      for (int c = 0; c < NC; ++c) {
-        xs[m][c] = ld(Xk + (m * NC + c) * V + s);
-        ysup[m][c] = ld(Yk + (m * NC + c) * V + y);
-      }
-    Mat<NC> A = mzero<NC>(), B = mzero<NC>();
-    lie_term<ND, NC, HERM>(mu, u, xs, ysup, A, B);
-    if (symmetric) {
-#pragma unroll
-      for (int m = 0; m < NS; ++m)
-#pragma unroll
-        for (int c = 0; c < NC; ++c) {
-          xs[m][c] = ld(Yk + (m * NC + c) * V + s);
-          ysup[m][c] = ld(Xk + (m * NC + c) * V + y);
-        }
-      lie_term<ND, NC, HERM>(mu, u, xs, ysup, A, B);
-    }
     const double w = 0.5 * kappa * terms.alpha[k];
-    cx<double> tr = (1.0 / NC) * (trace(A) - trace(B));
+    for (int side = 0; side < (symmetric ? 2 : 1); ++side) {
+      const double2* P = (side == 0 ? X : Y) + k * vec;  // L(P, Q): P at x, Q at x + mu
+      const double2* Q = (side == 0 ? Y : X) + k * vec;
 #pragma unroll
-    for (int uu = 0; uu < NC; ++uu)
+      for (int c = 0; c < (HERM ? NS / 2 : NS); ++c) {
+        const bool plus = c >= NS / 2;  // the B term of the plain projector
+        const int a = plus ? c - NS / 2 : c;
+        cx<double> h[NC], q[NC];
+        half_row<ND, NC>(P, mu, a, HERM || plus, V, s, h);
+        half_row<ND, NC>(Q, mu, a, plus, V, y, q);
+        const double wc = plus ? -w : w;
 #pragma unroll
-      for (int tt = 0; tt < NC; ++tt) {
-        cx<double> v = A.m[tt][uu] - B.m[tt][uu];
-        if (uu == tt) v -= tr;
-        F.m[uu][tt] += w * v;
+        for (int i = 0; i < NC; ++i) {
+          cx<double> v = u.m[i][0] * q[0];
+#pragma unroll
+          for (int l = 1; l < NC; ++l) cmac(v, u.m[i][l], q[l]);
+          v = wc * v;
+#pragma unroll
+          for (int j = 0; j < NC; ++j) {
+            if (plus) cmac_cj(K.m[i][j], v, h[j]);  // conj(v)_i x_j
+            else cmac_cj(K.m[j][i], h[j], v);       // conj(x)_j v_i
+          }
+        }
       }
+    }
   }
-  Mat<NC> out = load_link<NC>(force, mu, s, V);
+  if constexpr (HERM) {
+    Mat<NC> D;
+#pragma unroll
+    for (int i = 0; i < NC; ++i)
+#pragma unroll
+      for (int j = 0; j < NC; ++j) D.m[i][j] = K.m[i][j] - conj(K.m[j][i]);
+    K = D;
+  }
+  const cx<double> tr = (1.0 / NC) * trace(K);
+#pragma unroll
+  for (int i = 0; i < NC; ++i) K.m[i][i] -= tr;
 #pragma unroll
   for (int i = 0; i < NC; ++i)
 #pragma unroll
-    for (int j = 0; j < NC; ++j) out.m[i][j] += scale * F.m[i][j];
-  store_link<NC>(force, mu, s, V, out);
+    for (int j = 0; j < NC; ++j) {
+      double2* o = force + ((int64_t)(mu * NC + i) * NC + j) * V + s;
+      st(o, ld(o) + scale * K.m[j][i]);
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -796,7 +780,7 @@ int lym_fermion_force(const lym_lattice* lat, int nc, double kappa, int hermitia
   }
   ForceTerms t;
   for (int i = 0; i < kMaxForceTerms; ++i) t.alpha[i] = i < nterms ? alphas[i] : 0.0;
-  dim3 grid(grid_for(lat->V, 128), lat->nd);
+  const unsigned grid = warp_link_grid(lat->nd, lat->V, 128);
   cudaStream_t st = (cudaStream_t)stream;
   const int Lt = lat->dims[lat->nd - 1];
 #define LYM_FF(ND_, NC_, H_)                                                                        \
