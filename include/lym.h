@@ -308,6 +308,12 @@ int lym_gauge_hmc_step_multi(int nlat, const lym_lattice* const* lats, const int
                              void* const* gauges, void* const* momenta, double eps_p, double eps_u,
                              void* stream);
 
+/* One APE smearing step (smearing.py:34-51): out = P[(rho/6) S + (1 - rho) gauge] per link, S the
+ * staples without direction no_direction (-1: none), whose own links get rho U + (1 - rho) U,
+ * and P the projection of lym_unitary_projection.  out must not alias gauge. */
+int lym_ape_smear(const lym_lattice* lat, int nc, const void* gauge, double rho_re, double rho_im,
+                  int no_direction, void* out, void* stream);
+
 /* out = X (X^dag X)^{-1/2} / det^{1/N} per link (smearing.py:17-31). */
 int lym_unitary_projection(int nd, int nc, int64_t volume, const void* in, void* out, void* stream);
 
@@ -372,11 +378,22 @@ int lym_decode_xdr_gauge(int nd, int nc, int64_t volume, const void* raw, void* 
 int lym_path_product(const lym_lattice* lat, int nc, const void* gauge, int nsteps, const int* steps,
                      int trace, void* out, void* stream);
 
+/* plaquettes, squares (V) complex128: per site, the traces of the 1x1 and of the 2x2 loops
+ * starting there, summed over the planes without skip_direction (-1: all planes)
+ * (measurements.py:197-290). */
+int lym_plane_loops(const lym_lattice* lat, int nc, const void* gauge, int skip_direction, void* plaquettes,
+                    void* squares, void* stream);
+
 /* out (device, 2 L doubles, L = the extent of `direction`): out[2z], out[2z+1] = sum of the
  * complex field (V) over the sites with x_direction = z and, when mask_direction >= 0,
  * x_mask_direction = 0 (the zero-momentum projections of measurements.py:160-290). */
 int lym_slice_sums(const lym_lattice* lat, int direction, int mask_direction, const void* field,
                    double* out, void* stream);
+
+/* out (device, 2 L doubles, L = the extent of `direction`): out[2k], out[2k+1] = sum over the
+ * sites of conj(f(x + k)) f(x), f a complex128 field (V), x + k the site k steps forward in
+ * `direction` (the Polyakov-loop correlator of measurements.py:178-190). */
+int lym_shift_dots(const lym_lattice* lat, int direction, const void* field, double* out, void* stream);
 
 /* ------------------------------------------------------------------ */
 /* fermion measurements (fermion_measurements.py:41-115)               */

@@ -68,3 +68,92 @@ def test_adjoint_operator_and_force_on_ragged_lattices(cuda_device, geom, nc, un
             start = cnormal(rng, ref.shape)
             f = op.accumulate_force(cu(start), alphas, cu(x), cu(y), symmetric=symmetric, scale=0.5)
             assert relerr(f.cpu().numpy(), start + 0.5 * ref) < TOL, (herm, symmetric)
+
+
+@pytest.mark.parametrize("geom,nc,unitary", [((5, 7), 3, False), ((33, 1), 2, True), ((3, 2, 3, 5), 3, False),
+                                             ((1, 2, 4, 4), 2, True), ((3, 3, 1, 11), 3, True)])
+def test_fundamental_force_on_ragged_lattices(cuda_device, geom, nc, unitary):
+    rng = np.random.default_rng(int(np.prod(geom)) + nc)
+    nd, vol, kappa = len(geom), int(np.prod(geom)), 0.13
+    ns = 4 if nd == 4 else 2
+    u = links(rng, geom, nc, unitary)
+    tables, ubc = O.lookup_tables(geom), O.apply_time_bc(u, O.antiperiodic_field(geom, BC))
+    x, y = cnormal(rng, (3, ns, nc, vol)), cnormal(rng, (3, ns, nc, vol))
+    alphas = [0.7, -1.3, 0.2]
+    for herm in (False, True):
+        op = make_op(u, geom, kappa, herm, "fundamental")
+        for symmetric in (False, True):
+            ref = np.zeros((nd, nc, nc, vol), complex)
+            for k, a in enumerate(alphas):
+                ref += a * O.lie_derivative(ubc, x[k], y[k], kappa, herm, tables)
+                if symmetric:
+                    ref += a * O.lie_derivative(ubc, y[k], x[k], kappa, herm, tables)
+            start = cnormal(rng, ref.shape)
+            f = op.accumulate_force(cu(start), alphas, cu(x), cu(y), symmetric=symmetric, scale=0.5)
+            assert relerr(f.cpu().numpy(), start + 0.5 * ref) < TOL, (herm, symmetric)
+
+
+GEOMETRIES = [(7, 3), (2, 37), (3, 5, 2), (3, 1, 5, 7), (4, 3, 2, 33)]
+
+
+@pytest.mark.parametrize("geom", GEOMETRIES)
+@pytest.mark.parametrize("nc", [2, 3])
+def test_plaquette_staples_and_paths_on_ragged_lattices(cuda_device, geom, nc):
+    from tfleonardym_b200 import gauge_action, measurements, staples
+    from tfleonardym_b200 import lattice as lt
+    rng = np.random.default_rng(int(np.prod(geom)) * nc)
+    nd = len(geom)
+    u = links(rng, geom, nc, unitary=False)
+    tables = O.lookup_tables(geom)
+    cfg = lt.Configuration(cu(u), geom, nc, nd)
+    re, im = gauge_action.plaquette_trace_sum(cfg)
+    ref = O.plaquette_trace_sum(u, tables)
+    assert abs(complex(re, im) - ref) < TOL * np.sum(np.abs(u) ** 4)
+    for nodir in [-1] + list(range(nd)):
+        st = staples.get_staple_sums(cfg, nodir).cpu().numpy()
+        assert relerr(st, O.staples(u, tables, nodir if nodir >= 0 else None)) < TOL
+    f = gauge_action.yang_mills(cfg, 5.5).force().cpu().numpy()
+    assert relerr(f, O.gauge_force(u, 5.5, tables)) < TOL
+    # unit-size links, so that no length of a path overflows its tolerance
+    u = links(rng, geom, nc)
+    cfg = lt.Configuration(cu(u), geom, nc, nd)
+    paths = [[], [1], [-2], [2, -1], [1, 2, -1, -2], [nd, nd, -1, nd, 2], [1] * geom[0], [nd] * geom[-1],
+             [nd] * (geom[-1] + 1), [-nd] * geom[-1]]
+    for steps in paths:
+        got = measurements.path_field(cfg, steps).cpu().numpy()
+        if steps:
+            assert relerr(got, O.path_trace(u, tables, steps)) < TOL * max(1, len(steps)), steps
+            m = measurements.path_field(cfg, steps, trace=False).cpu().numpy()
+            assert relerr(m, O.path_product(u, tables, steps)) < TOL * max(1, len(steps)), steps
+        else:
+            assert np.all(got == nc)
+
+
+@pytest.mark.parametrize("geom", GEOMETRIES + [(6, 8, 4, 10)])
+def test_slice_sums_and_shifted_products(cuda_device, geom):
+    from tfleonardym_b200 import _dev, _lib, measurements
+    from tfleonardym_b200 import lattice as lt
+    rng = np.random.default_rng(int(np.prod(geom)))
+    vol = int(np.prod(geom))
+    f = cnormal(rng, (vol,))
+    cfg = lt.Configuration(cu(links(rng, geom, 2)), geom, 2, len(geom))
+    grid = f.reshape(geom)
+    for d in range(len(geom)):
+        others = tuple(k for k in range(len(geom)) if k != d)
+        scale = TOL * np.sum(np.abs(f))
+        assert np.max(np.abs(measurements._slice_sums(cfg, cu(f), d) - grid.sum(axis=others))) < scale
+        for m in others:
+            ref = grid.take([0], axis=m).sum(axis=others)
+            assert np.max(np.abs(measurements._slice_sums(cfg, cu(f), d, m) - ref)) < scale
+        ref = np.array([np.vdot(np.roll(grid, -k, axis=d), grid) for k in range(geom[d])])
+        assert np.max(np.abs(measurements._shift_dots(cfg, cu(f), d) - ref)) < TOL * np.sum(np.abs(f) ** 2)
+        for adjoint in (0, 1):
+            v = cnormal(rng, (3, 2, 2, 2, vol)) if adjoint else cnormal(rng, (3, 2, 3, vol))
+            w = np.swapaxes(v, 2, 3) if adjoint else v
+            ref = (np.conj(v) * w).reshape((-1, vol)).sum(0).reshape(geom).sum(axis=others)
+            out = torch.empty(2 * geom[d], dtype=torch.float64, device="cuda")
+            x = cu(v)
+            _lib.check(_lib.lib().lym_timeslice_sums(lt.get_lattice(geom).handle, d, 3, 2, 2 if adjoint else 3, adjoint,
+                                                     _dev.ptr(x), _dev.ptr(out), _dev.stream()), "lym_timeslice_sums")
+            o = out.cpu().numpy()
+            assert np.max(np.abs(o[0::2] + 1j * o[1::2] - ref)) < TOL * np.sum(np.abs(v) ** 2)

@@ -86,6 +86,7 @@ SIGNATURES = {
     "lym_momenta_energy": (c_int, [c_int, c_int, c_int64, c_void_p, P(c_double), c_void_p]),
     "lym_update_momenta": (c_int, [c_int64, c_void_p, c_void_p, c_double, c_void_p]),
     "lym_update_links": (c_int, [c_int, c_int, c_int64, c_void_p, c_void_p, c_double, c_int, c_void_p]),
+    "lym_ape_smear": (c_int, [c_void_p, c_int, c_void_p, c_double, c_double, c_int, c_void_p, c_void_p]),
     "lym_unitary_projection": (c_int, [c_int, c_int, c_int64, c_void_p, c_void_p, c_void_p]),
     "lym_fermion_force": (c_int, [c_void_p, c_int, c_double, c_int, c_double, c_double, c_void_p, c_int,
                                   P(c_double), c_void_p, c_void_p, c_int, c_double, c_void_p, c_void_p]),
@@ -95,6 +96,8 @@ SIGNATURES = {
     "lym_decode_xdr_gauge": (c_int, [c_int, c_int, c_int64, c_void_p, c_void_p, c_void_p]),
     "lym_path_product": (c_int, [c_void_p, c_int, c_void_p, c_int, P(c_int), c_int, c_void_p, c_void_p]),
     "lym_slice_sums": (c_int, [c_void_p, c_int, c_int, c_void_p, c_void_p, c_void_p]),
+    "lym_plane_loops": (c_int, [c_void_p, c_int, c_void_p, c_int, c_void_p, c_void_p, c_void_p]),
+    "lym_shift_dots": (c_int, [c_void_p, c_int, c_void_p, c_void_p, c_void_p]),
     "lym_timeslice_sums": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p]),
     "lym_fermion_force_adjoint": (c_int, [c_void_p, c_int, c_double, c_int, c_double, c_double, c_void_p, c_int,
                                           P(c_double), c_void_p, c_void_p, c_int, c_double, c_void_p,

@@ -150,28 +150,42 @@ __global__ void __launch_bounds__(128, 3) gauge_force_kernel(const int32_t* __re
 }
 
 // sum_{x, mu<nu} Tr U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag (gauge_action.py:110-113)
+// A warp takes one plane of 32 sites, the planes of a site block side by side (their 24
+// links in 4D are 16 distinct ones), and streams the rows of both half loops into the
+// trace.  24^3 x 48 SU(3): 162 us against 195 us with a thread doing all planes of a
+// site (255 registers).
 template <int ND, int NC>
-__global__ void __launch_bounds__(256) plaquette_kernel(const int32_t* __restrict__ tab, int64_t V,
-                                                        const double2* __restrict__ U, double* partials,
-                                                        unsigned* counter, double* result) {
+__global__ void __launch_bounds__(256, 2) plaquette_kernel(const int32_t* __restrict__ tab, int64_t V,
+                                                           const double2* __restrict__ U, double* partials,
+                                                           unsigned* counter, double* result) {
   __shared__ double sh[2 * 32];
+  constexpr int NP = ND * (ND - 1) / 2;
   double v[2] = {0.0, 0.0};
-  for (int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; s < V; s += (int64_t)gridDim.x * blockDim.x) {
+  const int64_t nw = (V + 31) / 32 * NP;
+  const int64_t per = (nw + gridDim.x - 1) / gridDim.x;  // a block's warps: a contiguous run of planes
+  const int64_t w1 = (blockIdx.x + 1) * per < nw ? (blockIdx.x + 1) * per : nw;
+  for (int64_t w = blockIdx.x * per + (threadIdx.x >> 5); w < w1; w += 8) {
+    const int64_t sb = w / NP;
+    int mu = 0, nu = (int)(w - sb * NP) + 1;
+    while (nu >= ND) nu += ++mu + 1 - ND;  // plane index -> mu < nu
+    const int64_t s = sb * 32 + (threadIdx.x & 31);
+    if (s >= V) continue;
+    const Mat<NC> b = load_link<NC>(U, nu, tab[mu * V + s], V), d = load_link<NC>(U, mu, tab[nu * V + s], V);
 #pragma unroll
-    for (int mu = 0; mu < ND; ++mu)
+    for (int i = 0; i < NC; ++i) {
+      cx<double> p[NC], q[NC], r[NC];
 #pragma unroll
-      for (int nu = mu + 1; nu < ND; ++nu) {
-        Mat<NC> a = mul(load_link<NC>(U, mu, s, V), load_link<NC>(U, nu, tab[mu * V + s], V));
-        Mat<NC> b = mul(load_link<NC>(U, nu, s, V), load_link<NC>(U, mu, tab[nu * V + s], V));
-        // Tr(a b^dag)
-        cx<double> t = czero<double>();
+      for (int k = 0; k < NC; ++k) p[k] = ld(U + ((int64_t)(mu * NC + i) * NC + k) * V + s);
+      row_mul<NC>(q, p, b);
 #pragma unroll
-        for (int i = 0; i < NC; ++i)
+      for (int k = 0; k < NC; ++k) p[k] = ld(U + ((int64_t)(nu * NC + i) * NC + k) * V + s);
+      row_mul<NC>(r, p, d);
 #pragma unroll
-          for (int k = 0; k < NC; ++k) t += a.m[i][k] * conj(b.m[i][k]);
-        v[0] += t.re;
-        v[1] += t.im;
+      for (int k = 0; k < NC; ++k) {  // Tr (U_mu U_nu(x+mu)) (U_nu U_mu(x+nu))^dag
+        v[0] += q[k].re * r[k].re + q[k].im * r[k].im;
+        v[1] += q[k].im * r[k].re - q[k].re * r[k].im;
       }
+    }
   }
   if (grid_sum<2>(v, partials, counter, sh) && threadIdx.x == 0) {
     result[0] = v[0];
@@ -347,32 +361,43 @@ LYM_D Mat<3> expm(const Mat<3>& X) {
   return mscale(cx<double>{e * cs, e * sn}, R);
 }
 
+// |d|^(-1/N)
+template <int NC>
+LYM_D double inv_root(double d2) { return NC == 2 ? rsqrt(sqrt(d2)) : rcbrt(sqrt(d2)); }
+
 // Unitary polar factor by the scaled Newton iteration
 // U <- (g U + U^{-dag} / g) / 2, g = |det U|^{-1/N} (Higham, "Functions of
 // Matrices", sec. 8.6), then division by the principal det^{1/N}
 // (smearing.py:17-31 computes X (X^dag X)^{-1/2} / det^{1/N} via sqrtm).
+// The iteration converges quadratically, |U_{k+1} - U| <= |U_k - U|^2 / 2 near the end, so
+// a step of squared length 1e-17 leaves an error of 1e-17 and is the last.
 template <int NC>
 LYM_D Mat<NC> polar_su(const Mat<NC>& X) {
   Mat<NC> Uk = X;
+  cx<double> d = det(Uk);
   for (int it = 0; it < 40; ++it) {
-    cx<double> d = det(Uk);
-    double g = pow(sqrt(norm2(d)), -1.0 / NC);
-    Mat<NC> Z = mdag(inverse(Uk));
-    Mat<NC> Un;
+    const double d2 = norm2(d);
+    // the scale only speeds up the approach: near |det U| = 1 it is left at 1
+    const double g = fabs(d2 - 1.0) < 1e-2 ? 1.0 : inv_root<NC>(d2);
+    const double hg = 0.5 * g, hi = 0.5 / (g * d2);
+    const Mat<NC> C = cofactors(Uk);  // U^{-dag} = conj(C) / conj(d) = conj(C) d / |d|^2
+    const cx<double> w = hi * d;
     double diff = 0.0;
 #pragma unroll
     for (int i = 0; i < NC; ++i)
 #pragma unroll
       for (int j = 0; j < NC; ++j) {
-        Un.m[i][j] = 0.5 * (g * Uk.m[i][j] + (1.0 / g) * Z.m[i][j]);
-        diff += norm2(Un.m[i][j] - Uk.m[i][j]);
+        cx<double> n = cmul_cj(C.m[i][j], w);
+        n.re = fma(hg, Uk.m[i][j].re, n.re);
+        n.im = fma(hg, Uk.m[i][j].im, n.im);
+        diff += norm2(n - Uk.m[i][j]);
+        Uk.m[i][j] = n;
       }
-    Uk = Un;
-    if (diff < 1e-30) break;
+    d = det(Uk);
+    if (diff < 1e-17) break;
   }
-  cx<double> r = principal_root(det(Uk), NC);
-  cx<double> ir = cdiv(cx<double>{1.0, 0.0}, r);
-  return mscale(ir, Uk);
+  const cx<double> r = principal_root(d, NC);
+  return mscale(cdiv(cx<double>{1.0, 0.0}, r), Uk);
 }
 
 template <int NC>
@@ -398,6 +423,32 @@ __global__ void __launch_bounds__(128) unitary_projection_kernel(int64_t nlinks,
   const int mu = (int)(l / V);
   const int64_t s = l - mu * V;
   store_link<NC>(out, mu, s, V, polar_su<NC>(load_link<NC>(in, mu, s, V)));
+}
+
+// One APE smearing step (smearing.py:34-51) per link: the staples without direction no_dir,
+// the fat link (rho / 6) S + (1 - rho) U (rho U + (1 - rho) U for no_dir) and its projection,
+// so the staples and the fat links never reach memory.  FP64-bound (the projection).
+// 24^3 x 48 SU(3): 565 us against 1108 us in separate passes (staples, four scaled
+// sums with their copies, projection).
+template <int ND, int NC>
+__global__ void __launch_bounds__(128, 4) smear_kernel(const int32_t* __restrict__ tab, int64_t V,
+                                                       const double2* __restrict__ U, cx<double> rho, int no_dir,
+                                                       double2* __restrict__ out) {
+  int mu;
+  int64_t s;
+  if (!warp_link(ND, V, blockIdx.x, mu, s)) return;
+  const cx<double> one{1.0, 0.0};
+  Mat<NC> F;
+  if (mu == no_dir) {
+    F = mscale(rho, load_link<NC>(U, mu, s, V));
+  } else {
+    F = mscale(cx<double>{rho.re / 6, rho.im / 6}, staple_sum<ND, NC>(tab, V, U, mu, s, no_dir));
+  }
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+#pragma unroll
+    for (int j = 0; j < NC; ++j) cmac(F.m[i][j], one - rho, ld(U + ((int64_t)(mu * NC + i) * NC + j) * V + s));
+  store_link<NC>(out, mu, s, V, polar_su<NC>(F));
 }
 
 // ---------------------------------------------------------------------------
@@ -639,7 +690,7 @@ int lym_plaquette_sum(const lym_lattice* lat, int nc, const void* gauge, double*
   std::lock_guard<std::mutex> lk(host_reduce_mutex());
   const int slot = 1;
   cudaStream_t st = (cudaStream_t)stream;
-  unsigned nb = reduction_blocks(lat->V, 256);
+  unsigned nb = reduction_blocks((lat->V + 31) / 32 * 32 * (lat->nd * (lat->nd - 1) / 2), 256);
   double* part = s->partials + (size_t)slot * Scratch::kMaxBlocks * Scratch::kMaxVals;
   double* res = s->results + slot * Scratch::kMaxVals;
   LYM_DISPATCH_ND_NC(lat->nd, nc, (plaquette_kernel<ND, NC><<<nb, 256, 0, st>>>(
@@ -751,6 +802,19 @@ int lym_update_links(int nd, int nc, int64_t volume, void* gauge, const void* mo
   return LYM_OK;
 }
 
+int lym_ape_smear(const lym_lattice* lat, int nc, const void* gauge, double rho_re, double rho_im, int no_direction,
+                  void* out, void* stream) {
+  LYM_REQUIRE(lat && gauge && out, LYM_ERR_BAD_ARG, "null argument");
+  LYM_REQUIRE(gauge != out, LYM_ERR_BAD_ARG, "gauge and out must not alias");
+  const unsigned grid = warp_link_grid(lat->nd, lat->V, 128);
+  cudaStream_t st = (cudaStream_t)stream;
+  LYM_DISPATCH_ND_NC(lat->nd, nc, (smear_kernel<ND, NC><<<grid, 128, 0, st>>>(
+                                      lat->d_tab, lat->V, (const double2*)gauge, cx<double>{rho_re, rho_im},
+                                      no_direction, (double2*)out)));
+  LYM_CHECK_LAUNCH();
+  return LYM_OK;
+}
+
 int lym_unitary_projection(int nd, int nc, int64_t volume, const void* in, void* out, void* stream) {
   LYM_REQUIRE(in && out && nd >= 1 && nd <= LYM_MAX_ND && volume >= 0, LYM_ERR_BAD_ARG, "bad argument");
   if (volume == 0) return LYM_OK;
@@ -808,30 +872,53 @@ int lym_fermion_force(const lym_lattice* lat, int nc, double kappa, int hermitia
 // ---------------------------------------------------------------------------
 namespace lym {
 
+static int64_t lat_stride(const lym_lattice* lat, int d) {
+  int64_t s = 1;
+  for (int e = d + 1; e < lat->nd; ++e) s *= lat->dims[e];
+  return s;
+}
+
 constexpr int kMaxPathSteps = 256;
 struct PathSteps {
   signed char step[kMaxPathSteps];  // +(mu+1): U_mu(y), y += mu;  -(mu+1): y -= mu, U_mu(y)^dag
 };
 
 // One thread per starting site: M = product of the links along the path; writes
-// Tr M (trace = 1, out (V) complex) or M (out (N, N, V)).
+// Tr M (trace = 1, out (V) complex) or M (out (N, N, V)).  The first link is taken as it
+// is and the last one enters the trace directly (n - 2 products and a trace for n links).
+// Bound by the latency of its dependent gathers: occupancy counts, so one link is held
+// at a time.  24^3 x 48 SU(3): 4 links 49 us against 54 us, 8 links 74 us against 84 us.
 template <int NC>
 __global__ void __launch_bounds__(128) path_kernel(const int32_t* __restrict__ tab, int nd, int64_t V,
                                                    const double2* __restrict__ U, int nsteps, PathSteps path,
                                                    int want_trace, double2* __restrict__ out) {
   const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (x >= V) return;
-  Mat<NC> m = mident<NC>();
   int64_t y = x;
+  Mat<NC> m = mident<NC>();
   for (int k = 0; k < nsteps; ++k) {
     const int s = path.step[k];
     const int mu = (s > 0 ? s : -s) - 1;
-    if (s > 0) {
-      m = mul(m, load_link<NC>(U, mu, y, V));
-      y = tab[mu * V + y];
+    const int64_t nx = tab[(s > 0 ? mu : nd + mu) * V + y];
+    const Mat<NC> l = load_link<NC>(U, mu, s > 0 ? y : nx, V);  // U_mu(y), or U_mu(y - mu) entering as its dagger
+    y = nx;
+    if (k == 0) {
+      m = s > 0 ? l : mdag(l);
+    } else if (want_trace && k == nsteps - 1) {
+      cx<double> t = czero<double>();
+#pragma unroll
+      for (int i = 0; i < NC; ++i)
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+          if (s > 0) cmac(t, m.m[i][j], l.m[j][i]);
+          else cmac_cj(t, l.m[i][j], m.m[i][j]);
+        }
+      st(out + x, t);
+      return;
+    } else if (s > 0) {
+      m = mul(m, l);
     } else {
-      y = tab[(nd + mu) * V + y];
-      m = mul_nd(m, load_link<NC>(U, mu, y, V));
+      m = mul_nd(m, l);
     }
   }
   if (want_trace) {
@@ -844,28 +931,140 @@ __global__ void __launch_bounds__(128) path_kernel(const int32_t* __restrict__ t
   }
 }
 
+// plaq(x), square(x) = sum over the planes without direction `skip` of the traces of the
+// 1 x 1 and 2 x 2 loops from x (measurements.py:197-290), each loop as its two halves
+// (Tr P Q^dag), all planes of a site in one thread: ten distinct links per plane, no
+// per-plane fields.  24^3 x 48 SU(3), three planes: 248 us against 1130 us for the six paths and
+// their sums.
+template <int NC>
+__global__ void __launch_bounds__(128, 3) plane_loops_kernel(const int32_t* __restrict__ tab, int nd, int64_t V,
+                                                             const double2* __restrict__ U, int skip,
+                                                             double2* __restrict__ plaq, double2* __restrict__ square) {
+  const int64_t x = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (x >= V) return;
+  cx<double> tp = czero<double>(), ts = czero<double>();
+#pragma unroll 1
+  for (int a = 0; a < nd; ++a)
+#pragma unroll 1
+    for (int b = a + 1; b < nd; ++b) {
+      if (a == skip || b == skip) continue;
+      const int64_t xa = tab[a * V + x], xb = tab[b * V + x], xaa = tab[a * V + xa], xbb = tab[b * V + xb];
+      const int64_t xaab = tab[b * V + xaa], xbba = tab[a * V + xbb];
+      {
+        const Mat<NC> b1 = load_link<NC>(U, b, xa, V), c1 = load_link<NC>(U, a, xb, V);
+#pragma unroll
+        for (int i = 0; i < NC; ++i) {
+          cx<double> p[NC], q[NC], r[NC];
+#pragma unroll
+          for (int k = 0; k < NC; ++k) p[k] = ld(U + ((int64_t)(a * NC + i) * NC + k) * V + x);
+          row_mul<NC>(q, p, b1);
+#pragma unroll
+          for (int k = 0; k < NC; ++k) p[k] = ld(U + ((int64_t)(b * NC + i) * NC + k) * V + x);
+          row_mul<NC>(r, p, c1);
+#pragma unroll
+          for (int k = 0; k < NC; ++k) cmac_cj(tp, r[k], q[k]);
+        }
+      }
+      Mat<NC> p = mul(load_link<NC>(U, a, x, V), load_link<NC>(U, a, xa, V));
+      p = mul(p, load_link<NC>(U, b, xaa, V));
+      p = mul(p, load_link<NC>(U, b, xaab, V));
+      Mat<NC> q = mul(load_link<NC>(U, b, x, V), load_link<NC>(U, b, xb, V));
+      q = mul(q, load_link<NC>(U, a, xbb, V));
+      const Mat<NC> l = load_link<NC>(U, a, xbba, V);
+#pragma unroll
+      for (int i = 0; i < NC; ++i) {
+        cx<double> r[NC];
+        row_mul<NC>(r, q.m[i], l);
+#pragma unroll
+        for (int k = 0; k < NC; ++k) cmac_cj(ts, r[k], p.m[i][k]);
+      }
+    }
+  st(plaq + x, tp);
+  st(square + x, ts);
+}
+
+// Trace of the links once around direction d: by the cyclic invariance of the trace it is
+// the same from every site of a line, so a line is multiplied once -- kPolySeg threads
+// each take a segment -- and its trace written to all of its sites, where the general
+// path multiplies the line from each of its L_d sites.  24^3 x 48 SU(3), 48 links:
+// 31 us against 319 us.
+constexpr int kPolySeg = 4;
+template <int NC>
+__global__ void __launch_bounds__(32 * kPolySeg) loop_kernel(int64_t nlines, int64_t V, int64_t stride, int L,
+                                                             int mu, const double2* __restrict__ U,
+                                                             double2* __restrict__ out) {
+  __shared__ cx<double> part[kPolySeg][NC * NC][32];
+  __shared__ cx<double> tr[32];
+  const int tx = threadIdx.x & 31, seg = threadIdx.x >> 5;
+  const int64_t line = blockIdx.x * (int64_t)32 + tx;
+  // line -> its first site: coordinates slower than d, then the faster ones
+  const int64_t x0 = line / stride * (stride * L) + line % stride;
+  const int q = (L + kPolySeg - 1) / kPolySeg, k0 = seg * q, k1 = k0 + q < L ? k0 + q : L;
+  Mat<NC> m = mident<NC>();
+  if (line < nlines && k0 < k1) {
+    m = load_link<NC>(U, mu, x0 + k0 * stride, V);
+    for (int k = k0 + 1; k < k1; ++k) m = mul(m, load_link<NC>(U, mu, x0 + k * stride, V));
+  }
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+#pragma unroll
+    for (int j = 0; j < NC; ++j) part[seg][i * NC + j][tx] = m.m[i][j];
+  __syncthreads();
+  if (seg == 0) {
+    for (int g = 1; g < kPolySeg; ++g) {
+      Mat<NC> n;
+#pragma unroll
+      for (int i = 0; i < NC; ++i)
+#pragma unroll
+        for (int j = 0; j < NC; ++j) n.m[i][j] = part[g][i * NC + j][tx];
+      m = mul(m, n);
+    }
+    tr[tx] = trace(m);
+  }
+  __syncthreads();
+  if (line < nlines)
+    for (int k = k0; k < k1; ++k) st(out + x0 + k * stride, tr[tx]);
+}
+
 // out[2z], out[2z+1] = sum of f(x) over the sites with x_dir = z (and, when
 // mask_len > 0, x_mask = 0); x_d = (x / stride_d) mod L_d for the lexicographic
-// index with the last coordinate fastest.  One block per slice, fixed-order
-// reduction (deterministic).
-__global__ void __launch_bounds__(256) slice_sum_kernel(int64_t V, int64_t stride, int L, int64_t mask_stride,
-                                                        int mask_len, const double2* __restrict__ f,
-                                                        double* __restrict__ out) {
-  __shared__ double sh[2 * 32];
-  const int z = blockIdx.x;
+// index with the last coordinate fastest.  The cluster walks its slice's sites only
+// (24^3 x 48: 5.4 us against 712 us for one block per slice that tested every site of
+// the lattice).
+__global__ void __cluster_dims__(kSliceCtas, 1, 1) __launch_bounds__(kSliceThreads)
+    slice_sum_kernel(uint32_t per, uint32_t stride, uint32_t L, uint32_t mask_stride, uint32_t mask_len,
+                     const double2* __restrict__ f, double* __restrict__ out) {
+  const uint32_t z = blockIdx.x / kSliceCtas, rank = blockIdx.x % kSliceCtas;
   double re = 0.0, im = 0.0;
-  for (int64_t x = threadIdx.x; x < V; x += blockDim.x) {
-    if ((x / stride) % L != z) continue;
+  for (uint32_t j = rank * kSliceThreads + threadIdx.x; j < per; j += kSliceCtas * kSliceThreads) {
+    const uint32_t x = (j / stride) * (L * stride) + z * stride + j % stride;
     if (mask_len > 0 && (x / mask_stride) % mask_len != 0) continue;
     const double2 v = f[x];
     re += v.x;
     im += v.y;
   }
-  double v2[2] = {re, im};
-  block_sum<2>(v2, sh);
-  if (threadIdx.x == 0) {
-    out[2 * z] = v2[0];
-    out[2 * z + 1] = v2[1];
+  cluster_pair_sum(re, im, out + 2 * z);
+}
+
+// out[2k], out[2k+1] = sum_x conj(f(x + k dir)) f(x) for k = 0 .. L/2, and the complex
+// conjugate for L - k (substitute x -> x - k): a cluster per k.
+__global__ void __cluster_dims__(kSliceCtas, 1, 1) __launch_bounds__(kSliceThreads)
+    shift_dots_kernel(uint32_t V, uint32_t stride, uint32_t L, const double2* __restrict__ f,
+                      double* __restrict__ out) {
+  const uint32_t k = blockIdx.x / kSliceCtas, rank = blockIdx.x % kSliceCtas;
+  double re = 0.0, im = 0.0;
+#pragma unroll 4
+  for (uint32_t x = rank * kSliceThreads + threadIdx.x; x < V; x += kSliceCtas * kSliceThreads) {
+    const uint32_t z = (x / stride) % L;
+    const uint32_t y = z + k < L ? x + k * stride : x - (L - k) * stride;
+    const double2 a = f[y], b = f[x];
+    re += a.x * b.x + a.y * b.y;
+    im += a.x * b.y - a.y * b.x;
+  }
+  cluster_pair_sum(re, im, out + 2 * k);
+  if (rank == 0 && threadIdx.x == 0 && k > 0 && L - k != k) {
+    out[2 * (L - k)] = out[2 * k];
+    out[2 * (L - k) + 1] = -out[2 * k + 1];
   }
 }
 
@@ -884,6 +1083,22 @@ extern "C" int lym_path_product(const lym_lattice* lat, int nc, const void* gaug
   }
   dim3 grid(grid_for(lat->V, 128));
   cudaStream_t st = (cudaStream_t)stream;
+  // once around one direction: the trace is the same along the line
+  const int d = nsteps > 0 ? steps[0] - 1 : -1;
+  bool around = trace && d >= 0 && nsteps == lat->dims[d];
+  for (int k = 1; k < nsteps && around; ++k) around = steps[k] == steps[0];
+  if (around && (nc == 2 || nc == 3)) {
+    const int64_t nlines = lat->V / nsteps;
+    const unsigned lg = grid_for(nlines, 32);
+    if (nc == 2)
+      loop_kernel<2><<<lg, 32 * kPolySeg, 0, st>>>(nlines, lat->V, lat_stride(lat, d), nsteps, d, (const double2*)gauge,
+                                                   (double2*)out);
+    else
+      loop_kernel<3><<<lg, 32 * kPolySeg, 0, st>>>(nlines, lat->V, lat_stride(lat, d), nsteps, d, (const double2*)gauge,
+                                                   (double2*)out);
+    LYM_CHECK_LAUNCH();
+    return LYM_OK;
+  }
   if (nc == 2)
     path_kernel<2><<<grid, 128, 0, st>>>(lat->d_tab, lat->nd, lat->V, (const double2*)gauge, nsteps, p, trace != 0,
                                          (double2*)out);
@@ -898,22 +1113,45 @@ extern "C" int lym_path_product(const lym_lattice* lat, int nc, const void* gaug
   return LYM_OK;
 }
 
+extern "C" int lym_plane_loops(const lym_lattice* lat, int nc, const void* gauge, int skip_direction, void* plaquettes,
+                               void* squares, void* stream) {
+  using namespace lym;
+  LYM_REQUIRE(lat && gauge && plaquettes && squares, LYM_ERR_BAD_ARG, "null argument");
+  LYM_REQUIRE(nc == 2 || nc == 3, LYM_ERR_UNSUPPORTED, "N=%d not supported", nc);
+  const unsigned grid = grid_for(lat->V, 128);
+  cudaStream_t st = (cudaStream_t)stream;
+  if (nc == 2)
+    plane_loops_kernel<2><<<grid, 128, 0, st>>>(lat->d_tab, lat->nd, lat->V, (const double2*)gauge, skip_direction,
+                                                (double2*)plaquettes, (double2*)squares);
+  else
+    plane_loops_kernel<3><<<grid, 128, 0, st>>>(lat->d_tab, lat->nd, lat->V, (const double2*)gauge, skip_direction,
+                                                (double2*)plaquettes, (double2*)squares);
+  LYM_CHECK_LAUNCH();
+  return LYM_OK;
+}
+
 extern "C" int lym_slice_sums(const lym_lattice* lat, int direction, int mask_direction, const void* field,
                               double* out, void* stream) {
   using namespace lym;
   LYM_REQUIRE(lat && field && out, LYM_ERR_BAD_ARG, "null argument");
   LYM_REQUIRE(direction >= 0 && direction < lat->nd && mask_direction < lat->nd, LYM_ERR_BAD_ARG,
               "direction out of range");
-  auto stride_of = [&](int d) {
-    int64_t s = 1;
-    for (int e = d + 1; e < lat->nd; ++e) s *= lat->dims[e];
-    return s;
-  };
   const int L = lat->dims[direction];
   const int mask_len = mask_direction >= 0 ? lat->dims[mask_direction] : 0;
-  slice_sum_kernel<<<L, 256, 0, (cudaStream_t)stream>>>(lat->V, stride_of(direction), L,
-                                                        mask_direction >= 0 ? stride_of(mask_direction) : 1,
-                                                        mask_len, (const double2*)field, out);
+  slice_sum_kernel<<<L * kSliceCtas, kSliceThreads, 0, (cudaStream_t)stream>>>(
+      (uint32_t)(lat->V / L), (uint32_t)lat_stride(lat, direction), L,
+      (uint32_t)(mask_direction >= 0 ? lat_stride(lat, mask_direction) : 1), mask_len, (const double2*)field, out);
+  LYM_CHECK_LAUNCH();
+  return LYM_OK;
+}
+
+extern "C" int lym_shift_dots(const lym_lattice* lat, int direction, const void* field, double* out, void* stream) {
+  using namespace lym;
+  LYM_REQUIRE(lat && field && out, LYM_ERR_BAD_ARG, "null argument");
+  LYM_REQUIRE(direction >= 0 && direction < lat->nd, LYM_ERR_BAD_ARG, "direction %d out of range", direction);
+  const int L = lat->dims[direction];
+  shift_dots_kernel<<<(L / 2 + 1) * kSliceCtas, kSliceThreads, 0, (cudaStream_t)stream>>>(
+      (uint32_t)lat->V, (uint32_t)lat_stride(lat, direction), L, (const double2*)field, out);
   LYM_CHECK_LAUNCH();
   return LYM_OK;
 }

@@ -1,5 +1,8 @@
-// Small SU(N) matrix algebra (N = 2, 3) in registers, FP64.
+// Small SU(N) matrix algebra (N = 2, 3) in registers, FP64, and what the per-link and
+// per-slice kernels share.
 #pragma once
+
+#include <cooperative_groups.h>
 
 #include "lym_internal.cuh"
 
@@ -189,31 +192,25 @@ LYM_D cx<double> det(const Mat<3>& a) {
          a.m[0][2] * (a.m[1][0] * a.m[2][1] - a.m[1][1] * a.m[2][0]);
 }
 
-// inverse via the adjugate
-LYM_D Mat<2> inverse(const Mat<2>& a) {
-  cx<double> d = det(a);
-  double n = norm2(d);
-  cx<double> id = {d.re / n, -d.im / n};
+// cofactor matrix C: inverse(A) = C^T / det(A)
+LYM_D Mat<2> cofactors(const Mat<2>& a) {
   Mat<2> r;
-  r.m[0][0] = id * a.m[1][1];
-  r.m[0][1] = -(id * a.m[0][1]);
-  r.m[1][0] = -(id * a.m[1][0]);
-  r.m[1][1] = id * a.m[0][0];
+  r.m[0][0] = a.m[1][1];
+  r.m[0][1] = -a.m[1][0];
+  r.m[1][0] = -a.m[0][1];
+  r.m[1][1] = a.m[0][0];
   return r;
 }
-LYM_D Mat<3> inverse(const Mat<3>& a) {
-  cx<double> d = det(a);
-  double n = norm2(d);
-  cx<double> id = {d.re / n, -d.im / n};
+LYM_D Mat<3> cofactors(const Mat<3>& a) {
   Mat<3> r;
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
     for (int j = 0; j < 3; ++j) {
-      // cofactor C_ji for r[i][j]
-      const int j1 = (j + 1) % 3, j2 = (j + 2) % 3, i1 = (i + 1) % 3, i2 = (i + 2) % 3;
-      cx<double> c = a.m[j1][i1] * a.m[j2][i2] - a.m[j1][i2] * a.m[j2][i1];
-      r.m[i][j] = id * c;
+      const int i1 = (i + 1) % 3, i2 = (i + 2) % 3, j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+      cx<double> t = a.m[i1][j1] * a.m[i2][j2];
+      cmac(t, -a.m[i1][j2], a.m[i2][j1]);
+      r.m[i][j] = t;
     }
   return r;
 }
@@ -231,6 +228,37 @@ LYM_D cx<double> principal_root(cx<double> z, int n) {
 LYM_D cx<double> cdiv(cx<double> a, cx<double> b) {
   double n = norm2(b);
   return {(a.re * b.re + a.im * b.im) / n, (a.im * b.re - a.re * b.im) / n};
+}
+
+// Sums over lattice slices and shifted products, a cluster of kSliceCtas blocks per sum:
+// every block adds its part in a fixed order, block 0 of the cluster adds the parts in
+// block order through distributed shared memory, so the result is deterministic and needs
+// no scratch that two streams could share.
+constexpr int kSliceCtas = 8, kSliceThreads = 512;
+
+LYM_D void cluster_pair_sum(double re, double im, double* out) {
+  __shared__ double sh[2 * 32];
+  __shared__ double mine[2];
+  double v[2] = {re, im};
+  block_sum<2>(v, sh);
+  if (threadIdx.x == 0) {
+    mine[0] = v[0];
+    mine[1] = v[1];
+  }
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
+  cl.sync();
+  if (cl.block_rank() == 0 && threadIdx.x == 0) {
+    double a = 0.0, b = 0.0;
+    for (int r = 0; r < kSliceCtas; ++r) {
+      const double* o = cl.map_shared_rank(mine, r);
+      a += o[0];
+      b += o[1];
+    }
+    out[0] = a;
+    out[1] = b;
+  }
+  cl.sync();  // no block leaves while its part may still be read
 }
 
 }  // namespace lym

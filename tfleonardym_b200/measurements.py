@@ -1,8 +1,9 @@
 """Gauge measurements (mirror of the reference's measurements.py on the GPU).
 
 Every observable is a trace of a link product along a closed path: the products
-run in lym_path_product (one thread per starting site), the sums over slices in
-lym_slice_sums and the totals in lym_cdot / lym_plaquette_sum.  Signatures,
+run in lym_path_product (one thread per starting site) and lym_plane_loops (the
+glueball operators), the sums over slices in lym_slice_sums, the shifted products of
+the Polyakov correlator in lym_shift_dots and the totals in lym_cdot / lym_plaquette_sum.  Signatures,
 orders and normalisations are the reference's (measurements.py:22-290).
 """
 import ctypes
@@ -58,6 +59,16 @@ def _slice_sums(cfg, field, direction, mask_direction=-1):
     return o[0::2] + 1j * o[1::2]
 
 
+def _shift_dots(cfg, field, direction):
+    """sum_x conj(field(x + k direction)) field(x) for every k, as a complex numpy array."""
+    length = cfg.geometry[direction]
+    out = torch.empty(2 * length, dtype=torch.float64, device=field.device)
+    _lib.check(_lib.lib().lym_shift_dots(_lattice(cfg).handle, int(direction), _dev.ptr(_dev.as_c128(field)),
+                                         _dev.ptr(out), _dev.stream()), "lym_shift_dots")
+    o = out.cpu().numpy()
+    return o[0::2] + 1j * o[1::2]
+
+
 def temporal_plaquette(cfg) -> Measurement:
     """measurements.py:46-66."""
     nd, nc, vol = cfg.gauge_field.shape[0], cfg.gauge_field.shape[1], cfg.gauge_field.shape[-1]
@@ -99,11 +110,7 @@ def polyakov_operators(cfg, correlator_direction=2, polyakov_direction=3):
     meson = p * torch.conj(lt.mth_translate(p, 1, +1, lat))
     count = vol // (cfg.geometry[correlator_direction] * cfg.geometry[polyakov_direction])
     mz = _slice_sums(cfg, meson, correlator_direction, polyakov_direction) / count
-    corr = []
-    pdt = p
-    for _ in range(cfg.geometry[correlator_direction]):
-        corr.append(_dev.cdot(pdt, p) / vol)  # mean of p * conj(p_dt)
-        pdt = lt.mth_translate(pdt, correlator_direction, +1, lat)
+    corr = list(_shift_dots(cfg, p, correlator_direction) / vol)  # means of p * conj(p_dt)
     return [Measurement(name="meson_operator", value=np.array(mz), geometry=cfg.geometry, colors=cfg.colors),
             Measurement(name="polyakov_correlator", value=np.array(corr), geometry=cfg.geometry, colors=cfg.colors),
             Measurement(name="polyakov_loop", value=_total(p) / vol, geometry=cfg.geometry, colors=cfg.colors)]
@@ -113,17 +120,13 @@ def glueball_operators(cfg, correlator_direction=2):
     """Per-slice means of the summed 1x1 plaquette and 2x2 square traces over the planes
     without `correlator_direction` (measurements.py:197-290)."""
     nd, vol = cfg.gauge_field.shape[0], cfg.gauge_field.shape[-1]
-    plaq = None
-    square = None
-    for mu in range(nd):
-        for nu in range(mu + 1, nd):
-            if correlator_direction in (mu, nu):
-                continue
-            a, b = mu + 1, nu + 1
-            p1 = path_field(cfg, [a, b, -a, -b])
-            s1 = path_field(cfg, [a, a, b, b, -a, -a, -b, -b])
-            plaq = p1 if plaq is None else plaq + p1
-            square = s1 if square is None else square + s1
+    if nd == 2 and correlator_direction in (0, 1):
+        raise TypeError("two dimensions have no plane without the correlator direction")
+    u = _dev.as_c128(cfg.gauge_field)
+    plaq = torch.empty(vol, dtype=torch.complex128, device=u.device)
+    square = torch.empty_like(plaq)
+    _lib.check(_lib.lib().lym_plane_loops(_lattice(cfg).handle, u.shape[1], _dev.ptr(u), int(correlator_direction),
+                                          _dev.ptr(plaq), _dev.ptr(square), _dev.stream()), "lym_plane_loops")
     count = vol // cfg.geometry[correlator_direction]
     pz = _slice_sums(cfg, plaq, correlator_direction) / count
     sz = _slice_sums(cfg, square, correlator_direction) / count
