@@ -296,6 +296,15 @@ int lym_update_momenta(int64_t n, void* momenta, const void* force, double eps, 
 int lym_update_links(int nd, int nc, int64_t volume, void* gauge, const void* momenta,
                      double eps, int reunitarize, void* stream);
 
+/* The same three updates into another buffer (out may also be the field that is updated), for
+ * callers whose update returns a new field, as the reference's do: out = momenta + eps * F_gauge,
+ * out = momenta + eps * force, out = expm(eps P) gauge. */
+int lym_gauge_kick(const lym_lattice* lat, int nc, double beta, const void* gauge, const void* momenta,
+                   double eps, void* out, void* stream);
+int lym_momenta_kick(int64_t n, const void* momenta, const void* force, double eps, void* out, void* stream);
+int lym_link_drift(int nd, int nc, int64_t volume, const void* gauge, const void* momenta, double eps,
+                   int reunitarize, void* out, void* stream);
+
 /* The gauge part of an HMC step on nlat independent lattices (each its own lattice
  * object, N, beta, links gauges[l] and momenta momenta[l], reference layout) in two
  * launches whatever their sizes and (nd, N): momenta += eps_p * F_gauge(U) for every

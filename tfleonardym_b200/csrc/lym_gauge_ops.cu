@@ -127,26 +127,30 @@ LYM_D Mat<NC> gauge_force_link(const int32_t* __restrict__ tab, int64_t V, const
 }
 
 // F = -beta/(4N) (W^dag - W) - trace/N, W = U S^dag (gauge_action.py:42-53).
-// With mom != null: mom += eps F instead of storing F (hmc.py:59-61).
+// With mom != null: out = mom + eps F instead of F (hmc.py:59-61); out may be mom (each
+// thread reads its own link's momenta and writes them).
 template <int ND, int NC>
 __global__ void __launch_bounds__(128, 3) gauge_force_kernel(const int32_t* __restrict__ tab, int64_t V,
                                                              const double2* __restrict__ U, double beta,
-                                                             double2* __restrict__ force, double2* __restrict__ mom,
-                                                             double eps) {
+                                                             const double2* mom, double2* out, double eps) {
   int mu;
   int64_t s;
   if (!warp_link(ND, V, blockIdx.x, mu, s)) return;
-  const Mat<NC> F = gauge_force_link<ND, NC>(tab, V, U, beta, mu, s);
+  Mat<NC> F = gauge_force_link<ND, NC>(tab, V, U, beta, mu, s);
   if (mom) {
-    Mat<NC> P = load_link<NC>(mom, mu, s, V);
+    Mat<NC> P;  // all of it before the first store: out may be mom
 #pragma unroll
-    for (int i = 0; i < NC; ++i)
+    for (int k = 0; k < NC * NC; ++k) {
+      const double2 p = mom[(int64_t)(mu * NC * NC + k) * V + s];
+      P.m[k / NC][k % NC] = {p.x, p.y};
+    }
 #pragma unroll
-      for (int j = 0; j < NC; ++j) P.m[i][j] += eps * F.m[i][j];
-    store_link<NC>(mom, mu, s, V, P);
-  } else {
-    store_link<NC>(force, mu, s, V, F);
+    for (int k = 0; k < NC * NC; ++k) {
+      cx<double>& f = F.m[k / NC][k % NC];
+      f = P.m[k / NC][k % NC] + eps * f;
+    }
   }
+  store_link<NC>(out, mu, s, V, F);
 }
 
 // sum_{x, mu<nu} Tr U_mu(x) U_nu(x+mu) U_mu(x+nu)^dag U_nu(x)^dag (gauge_action.py:110-113)
@@ -253,10 +257,11 @@ __global__ void __launch_bounds__(256) momenta_energy_kernel(int64_t nlinks, int
   if (grid_sum<1>(v, partials, counter, sh) && threadIdx.x == 0) result[0] = v[0];
 }
 
-__global__ void axpy_real_kernel(int64_t n, double2* __restrict__ y, const double2* __restrict__ x, double a) {
+// out = y + a x (out may be y)
+__global__ void axpy_real_kernel(int64_t n, const double2* y, const double2* __restrict__ x, double a, double2* out) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     double2 yv = y[i], xv = x[i];
-    y[i] = make_double2(yv.x + a * xv.x, yv.y + a * xv.y);
+    out[i] = make_double2(yv.x + a * xv.x, yv.y + a * xv.y);
   }
 }
 
@@ -271,6 +276,21 @@ LYM_D double sinc(double w) {
     return 1.0 - w2 / 6.0 * (1.0 - w2 / 20.0 * (1.0 - w2 / 42.0 * (1.0 - w2 / 72.0)));
   }
   return sin(w) / w;
+}
+
+// exp(t) of the trace part; momenta are traceless up to rounding, where four terms of the
+// series are exact to rounding (|t|^5 / 120 < 1e-17)
+LYM_D cx<double> exp_trace(cx<double> t) {
+  if (norm2(t) < 1e-8) {
+    cx<double> r = {1.0 + 0.25 * t.re, 0.25 * t.im};
+    r = cx<double>{1.0, 0.0} + (1.0 / 3.0) * (t * r);
+    r = cx<double>{1.0, 0.0} + 0.5 * (t * r);
+    return cx<double>{1.0, 0.0} + t * r;
+  }
+  const double e = exp(t.re);
+  double sn, cs;
+  sincos(t.im, &sn, &cs);
+  return {e * cs, e * sn};
 }
 
 // exp(X) for 2x2 X = t 1 + X0, X0 traceless: X0^2 = -det(X0) 1 (Cayley-Hamilton),
@@ -291,9 +311,7 @@ LYM_D Mat<2> expm(const Mat<2>& X) {
   R.m[0][0].re += c;
   R.m[1][1].re += c;
   // exp(t) with t = i phi for anti-Hermitian X (real part kept for generality)
-  double e = exp(t.re), sn, cs;
-  sincos(t.im, &sn, &cs);
-  return mscale(cx<double>{e * cs, e * sn}, R);
+  return mscale(exp_trace(t), R);
 }
 
 // exp(X) for 3x3 anti-Hermitian X: X = t 1 + i Q with Q Hermitian traceless,
@@ -322,18 +340,20 @@ LYM_D Mat<3> expm(const Mat<3>& X) {
     double c0 = det(Q).re;
     const bool neg = c0 < 0;
     if (neg) c0 = -c0;
-    const double c0max = 2.0 * pow(c1 / 3.0, 1.5);
+    const double c13 = c1 / 3.0, r13 = sqrt(c13);
+    const double c0max = 2.0 * c13 * r13;
     double ratio = c0 / c0max;
     ratio = fmin(1.0, fmax(-1.0, ratio));
     const double theta = acos(ratio);
     double st3, ct3;
     sincos(theta / 3.0, &st3, &ct3);
-    const double u = sqrt(c1 / 3.0) * ct3;
+    const double u = r13 * ct3;
     const double w = sqrt(c1) * st3;
     const double u2 = u * u, w2 = w * w;
     double s2u, c2u, su, cu;
-    sincos(2.0 * u, &s2u, &c2u);
     sincos(u, &su, &cu);
+    s2u = 2.0 * su * cu;
+    c2u = (cu - su) * (cu + su);
     const cx<double> e2iu{c2u, s2u}, emiu{cu, -su};
     const double cw = cos(w), xi0 = sinc(w);
     cx<double> h0 = (u2 - w2) * e2iu + emiu * cx<double>{8.0 * u2 * cw, 2.0 * u * (3.0 * u2 + w2) * xi0};
@@ -349,16 +369,21 @@ LYM_D Mat<3> expm(const Mat<3>& X) {
       f2 = conj(f2);
     }
   }
+  const cx<double> et = exp_trace(t);
+  f0 = et * f0;
+  f1 = et * f1;
+  f2 = et * f2;
   Mat<3> R;
 #pragma unroll
   for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int j = 0; j < 3; ++j) R.m[i][j] = f1 * Q.m[i][j] + f2 * Q2.m[i][j];
+    for (int j = 0; j < 3; ++j) {
+      R.m[i][j] = f1 * Q.m[i][j];
+      cmac(R.m[i][j], f2, Q2.m[i][j]);
+    }
 #pragma unroll
   for (int i = 0; i < 3; ++i) R.m[i][i] += f0;
-  double e = exp(t.re), sn, cs;
-  sincos(t.im, &sn, &cs);
-  return mscale(cx<double>{e * cs, e * sn}, R);
+  return R;
 }
 
 // |d|^(-1/N)
@@ -401,17 +426,28 @@ LYM_D Mat<NC> polar_su(const Mat<NC>& X) {
 }
 
 template <int NC>
-__global__ void __launch_bounds__(128) update_links_kernel(int64_t nlinks, int64_t V, double2* __restrict__ U,
-                                                           const double2* __restrict__ P, double eps, int reunit) {
+__global__ void __launch_bounds__(128) update_links_kernel(int64_t nlinks, int64_t V, const double2* U,
+                                                           const double2* __restrict__ P, double eps, int reunit,
+                                                           double2* out) {
   const int64_t l = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   if (l >= nlinks) return;
   const int mu = (int)(l / V);
   const int64_t s = l - mu * V;
-  Mat<NC> p = load_link<NC>(P, mu, s, V);
-  Mat<NC> e = expm(mscale(cx<double>{eps, 0.0}, p));
-  Mat<NC> r = mul(e, load_link<NC>(U, mu, s, V));
+  Mat<NC> p = load_link<NC>(P, mu, s, V), u;
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+#pragma unroll
+    for (int j = 0; j < NC; ++j) {
+      const double2 t = U[((int64_t)(mu * NC + i) * NC + j) * V + s];  // out may be U
+      u.m[i][j] = {t.x, t.y};
+    }
+#pragma unroll
+  for (int i = 0; i < NC; ++i)
+#pragma unroll
+    for (int j = 0; j < NC; ++j) p.m[i][j] = eps * p.m[i][j];
+  Mat<NC> r = mul(expm(p), u);
   if (reunit) r = polar_su<NC>(r);
-  store_link<NC>(U, mu, s, V, r);
+  store_link<NC>(out, mu, s, V, r);
 }
 
 template <int NC>
@@ -669,17 +705,29 @@ int lym_staples(const lym_lattice* lat, int nc, const void* gauge, int no_direct
   return LYM_OK;
 }
 
+// force: out = F; kick: out = mom + eps F
+static int gauge_force(const lym_lattice* lat, int nc, double beta, const void* gauge, const void* mom, void* out,
+                       double eps, cudaStream_t st) {
+  const unsigned grid = warp_link_grid(lat->nd, lat->V, 128);
+  LYM_DISPATCH_ND_NC(lat->nd, nc, (gauge_force_kernel<ND, NC><<<grid, 128, 0, st>>>(
+                                      lat->d_tab, lat->V, (const double2*)gauge, beta, (const double2*)mom,
+                                      (double2*)out, eps)));
+  LYM_CHECK_LAUNCH();
+  return LYM_OK;
+}
+
 int lym_gauge_force(const lym_lattice* lat, int nc, double beta, const void* gauge, void* force, void* momenta,
                     double eps, void* stream) {
   LYM_REQUIRE(lat && gauge && (force || momenta), LYM_ERR_BAD_ARG, "null argument");
   LYM_REQUIRE(gauge != force && gauge != momenta, LYM_ERR_BAD_ARG, "outputs must not alias the gauge field");
-  const unsigned grid = warp_link_grid(lat->nd, lat->V, 128);
-  cudaStream_t st = (cudaStream_t)stream;
-  LYM_DISPATCH_ND_NC(lat->nd, nc, (gauge_force_kernel<ND, NC><<<grid, 128, 0, st>>>(
-                                      lat->d_tab, lat->V, (const double2*)gauge, beta, (double2*)force,
-                                      (double2*)momenta, eps)));
-  LYM_CHECK_LAUNCH();
-  return LYM_OK;
+  return gauge_force(lat, nc, beta, gauge, momenta, momenta ? momenta : force, eps, (cudaStream_t)stream);
+}
+
+int lym_gauge_kick(const lym_lattice* lat, int nc, double beta, const void* gauge, const void* momenta, double eps,
+                   void* out, void* stream) {
+  LYM_REQUIRE(lat && gauge && momenta && out, LYM_ERR_BAD_ARG, "null argument");
+  LYM_REQUIRE(gauge != out, LYM_ERR_BAD_ARG, "out must not alias the gauge field");
+  return gauge_force(lat, nc, beta, gauge, momenta, out, eps, (cudaStream_t)stream);
 }
 
 int lym_plaquette_sum(const lym_lattice* lat, int nc, const void* gauge, double* out, void* stream) {
@@ -741,13 +789,17 @@ int lym_momenta_energy(int nd, int nc, int64_t volume, const void* momenta, doub
   return LYM_OK;
 }
 
-int lym_update_momenta(int64_t n, void* momenta, const void* force, double eps, void* stream) {
-  LYM_REQUIRE(n >= 0 && momenta && force, LYM_ERR_BAD_ARG, "null argument");
+int lym_momenta_kick(int64_t n, const void* momenta, const void* force, double eps, void* out, void* stream) {
+  LYM_REQUIRE(n >= 0 && momenta && force && out, LYM_ERR_BAD_ARG, "null argument");
   if (n == 0) return LYM_OK;
-  axpy_real_kernel<<<reduction_blocks(n, 256) * 4, 256, 0, (cudaStream_t)stream>>>(n, (double2*)momenta,
-                                                                                     (const double2*)force, eps);
+  axpy_real_kernel<<<reduction_blocks(n, 256) * 4, 256, 0, (cudaStream_t)stream>>>(
+      n, (const double2*)momenta, (const double2*)force, eps, (double2*)out);
   LYM_CHECK_LAUNCH();
   return LYM_OK;
+}
+
+int lym_update_momenta(int64_t n, void* momenta, const void* force, double eps, void* stream) {
+  return lym_momenta_kick(n, momenta, force, eps, momenta, stream);
 }
 
 int lym_gauge_hmc_step_multi(int nlat, const lym_lattice* const* lats, const int* nc, const double* betas,
@@ -782,24 +834,29 @@ int lym_gauge_hmc_step_multi(int nlat, const lym_lattice* const* lats, const int
   return LYM_OK;
 }
 
-int lym_update_links(int nd, int nc, int64_t volume, void* gauge, const void* momenta, double eps, int reunitarize,
-                     void* stream) {
-  LYM_REQUIRE(gauge && momenta && nd >= 1 && nd <= LYM_MAX_ND && volume >= 0, LYM_ERR_BAD_ARG, "bad argument");
+int lym_link_drift(int nd, int nc, int64_t volume, const void* gauge, const void* momenta, double eps,
+                   int reunitarize, void* out, void* stream) {
+  LYM_REQUIRE(gauge && momenta && out && nd >= 1 && nd <= LYM_MAX_ND && volume >= 0, LYM_ERR_BAD_ARG, "bad argument");
   if (volume == 0) return LYM_OK;
   const int64_t nl = (int64_t)nd * volume;
   cudaStream_t st = (cudaStream_t)stream;
   if (nc == 2)
-    update_links_kernel<2><<<grid_for(nl, 128), 128, 0, st>>>(nl, volume, (double2*)gauge,
-                                                              (const double2*)momenta, eps, reunitarize);
+    update_links_kernel<2><<<grid_for(nl, 128), 128, 0, st>>>(nl, volume, (const double2*)gauge,
+                                                              (const double2*)momenta, eps, reunitarize, (double2*)out);
   else if (nc == 3)
-    update_links_kernel<3><<<grid_for(nl, 128), 128, 0, st>>>(nl, volume, (double2*)gauge,
-                                                              (const double2*)momenta, eps, reunitarize);
+    update_links_kernel<3><<<grid_for(nl, 128), 128, 0, st>>>(nl, volume, (const double2*)gauge,
+                                                              (const double2*)momenta, eps, reunitarize, (double2*)out);
   else {
     set_error("N=%d not supported", nc);
     return LYM_ERR_UNSUPPORTED;
   }
   LYM_CHECK_LAUNCH();
   return LYM_OK;
+}
+
+int lym_update_links(int nd, int nc, int64_t volume, void* gauge, const void* momenta, double eps, int reunitarize,
+                     void* stream) {
+  return lym_link_drift(nd, nc, volume, gauge, momenta, eps, reunitarize, gauge, stream);
 }
 
 int lym_ape_smear(const lym_lattice* lat, int nc, const void* gauge, double rho_re, double rho_im, int no_direction,

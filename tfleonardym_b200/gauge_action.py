@@ -38,6 +38,15 @@ class yang_mills:  # noqa: N801 - reference name
                                               None, _dev.ptr(momenta), float(eps), _dev.stream()), "lym_gauge_force")
         return momenta
 
+    def kicked_momenta(self, momenta, eps):
+        """momenta + eps * force() as a new tensor, in one kernel."""
+        u = _dev.as_c128(self.cfg.gauge_field)
+        p = _dev.as_c128(momenta)
+        out = torch.empty_like(p)
+        _lib.check(_lib.lib().lym_gauge_kick(_lat(self.cfg).handle, u.shape[1], float(self.beta), _dev.ptr(u),
+                                             _dev.ptr(p), float(eps), _dev.ptr(out), _dev.stream()), "lym_gauge_kick")
+        return out
+
     def energy(self):
         re, _ = plaquette_trace_sum(self.cfg)
         return -self.beta * re / self.cfg.gauge_field.shape[1]

@@ -1,9 +1,9 @@
 """Hybrid Monte Carlo (mirror of the reference's hmc.py on the GPU).
 
 The per-link kernels replace the reference's TF ops: ``update_link_field``
-(hmc.py:40-43, tf.linalg.expm) runs lym_update_links (SU(2) closed form,
+(hmc.py:40-43, tf.linalg.expm) runs lym_link_drift (SU(2) closed form,
 SU(3) Cayley-Hamilton), ``update_momenta`` (hmc.py:59-61) runs
-lym_update_momenta, ``momenta_energy`` (hmc.py:170-176) lym_momenta_energy.
+lym_momenta_kick, ``momenta_energy`` (hmc.py:170-176) lym_momenta_energy.
 The integrators are compiled into flat schedules of drifts and kicks (below)
 and run over these device tensors; ``integrate_om`` / ``integrate_lp`` /
 ``hybrid_mc`` / ``reversibility_check`` keep the reference's signatures and
@@ -15,7 +15,7 @@ import ctypes
 import numpy as np
 import torch
 
-from . import _dev, _lib, lie_generators
+from . import _dev, _lib, gauge_action, lie_generators
 from . import lattice as lt
 from . import smearing
 
@@ -24,12 +24,13 @@ OMELYAN_LAMBDA = 0.19318332275037863
 
 def update_link_field(link_field, momenta, epsilon, reunitarize=False):
     """expm(eps P) U per link, as a new tensor (hmc.py:40-43)."""
-    u = _dev.as_c128(link_field).clone()
+    u = _dev.as_c128(link_field)
     p = _dev.as_c128(momenta)
-    _lib.check(_lib.lib().lym_update_links(u.shape[0], u.shape[1], u.shape[-1], _dev.ptr(u), _dev.ptr(p),
-                                           float(epsilon), int(bool(reunitarize)), _dev.stream()),
-               "lym_update_links")
-    return u
+    out = torch.empty_like(u)
+    _lib.check(_lib.lib().lym_link_drift(u.shape[0], u.shape[1], u.shape[-1], _dev.ptr(u), _dev.ptr(p),
+                                         float(epsilon), int(bool(reunitarize)), _dev.ptr(out), _dev.stream()),
+               "lym_link_drift")
+    return out
 
 
 def update_configuration(config: lt.Configuration, momenta, epsilon):
@@ -40,11 +41,12 @@ def update_configuration(config: lt.Configuration, momenta, epsilon):
 
 def update_momenta(momenta, gauge_force, epsilon):
     """P + eps F as a new tensor (hmc.py:59-61)."""
-    p = _dev.as_c128(momenta).clone()
+    p = _dev.as_c128(momenta)
     f = _dev.as_c128(gauge_force)
-    _lib.check(_lib.lib().lym_update_momenta(p.numel(), _dev.ptr(p), _dev.ptr(f), float(epsilon), _dev.stream()),
-               "lym_update_momenta")
-    return p
+    out = torch.empty_like(p)
+    _lib.check(_lib.lib().lym_momenta_kick(p.numel(), _dev.ptr(p), _dev.ptr(f), float(epsilon), _dev.ptr(out),
+                                           _dev.stream()), "lym_momenta_kick")
+    return out
 
 
 def momenta_from_normals(normals, nc):
@@ -219,6 +221,8 @@ def force_evaluations(ops):
 
 
 def _kick(action, momenta, w):
+    if type(action) is gauge_action.yang_mills:  # a subclass may have its own force_into_momenta
+        return action.kicked_momenta(momenta, w)
     fused = getattr(action, "force_into_momenta", None)
     if fused is not None:
         return fused(momenta.clone(), w)
