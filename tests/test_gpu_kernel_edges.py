@@ -157,3 +157,96 @@ def test_slice_sums_and_shifted_products(cuda_device, geom):
                                                      _dev.ptr(x), _dev.ptr(out), _dev.stream()), "lym_timeslice_sums")
             o = out.cpu().numpy()
             assert np.max(np.abs(o[0::2] + 1j * o[1::2] - ref)) < TOL * np.sum(np.abs(v) ** 2)
+
+
+def smooth_links(rng, geom, nc, spread=0.3):
+    x = spread * cnormal(rng, (len(geom), nc, nc, int(np.prod(geom))))
+    for i in range(nc):
+        x[:, i, i] += 1
+    return O.unitary_sqrt_projection(x)
+
+
+# sites per parity: one block of 64 (2, 8, 64) and of 256 threads (256), the first cluster
+# (272), full clusters of 128 (1024) and the first of 256 threads (1056), two sites per
+# thread (4096), and the last sizes of the rule (8192 in reduced precisions, 2D)
+SOLVE_SHAPES = [((2, 2), 2), ((2, 2, 2, 2), 3), ((8, 16), 3), ((16, 32), 2), ((16, 34), 2), ((32, 64), 2),
+                ((32, 66), 3), ((64, 128), 2), ((128, 128), 2), ((8, 8, 8), 2), ((6, 10, 10), 3), ((16, 16, 16), 2),
+                ((4, 4, 4, 8), 2), ((4, 4, 6, 8), 3), ((8, 8, 8, 8), 3)]
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32", "f16", "bf16"])
+@pytest.mark.parametrize("geom,nc", SOLVE_SHAPES)
+def test_solve_on_small_lattices(cuda_device, geom, nc, precision):
+    """True residuals by the oracle below the target; the solutions of the launch-per-kernel
+    form (a forced tile) to the accuracy both targets leave: each is within tol / s of the
+    exact one, s >= 0.2 the smallest singular value of D at this kappa, so 1e-9 apart."""
+    from tfleonardym_b200 import dirac_solver
+    rng = np.random.default_rng(int(np.prod(geom)) + nc)
+    nd, vol, kappa, tol = len(geom), int(np.prod(geom)), 0.11, 1e-10
+    ns = 4 if nd == 4 else 2
+    u = smooth_links(rng, geom, nc)
+    ubc, tables = O.apply_time_bc(u, O.antiperiodic_field(geom, BC)), O.lookup_tables(geom)
+    b = cnormal(rng, (3, ns, nc, vol))
+    for herm in ([False] if nd == 3 else [False, True]):
+        op = make_op(u, geom, kappa, herm, "fundamental")
+        solver = dirac_solver.conjugate_gradient(tol=tol, precision=precision, delta=0.05)
+        x = solver.solve(op, cu(b))
+        tiled = dirac_solver.conjugate_gradient(tol=tol, precision=precision, delta=0.05, rhs_per_thread=1)
+        y = tiled.solve(op, cu(b))
+        for i in range(3):
+            res = np.linalg.norm(b[i] - O.wilson_apply(ubc, x[i].cpu().numpy(), kappa, herm, tables))
+            assert res < tol * np.linalg.norm(b[i]), (herm, i, solver.reports[i])
+            assert solver.reports[i]["status"] == 0 and abs(solver.reports[i]["true_residual"] * np.linalg.norm(b[i])
+                                                            - res) < 0.01 * tol * np.linalg.norm(b[i])
+            assert relerr(x[i].cpu().numpy(), y[i].cpu().numpy()) < 10 * tol
+        alone = solver.solve(op, cu(b[1]))
+        assert relerr(alone.cpu().numpy(), x[1].cpu().numpy()) < 10 * tol
+
+
+def test_solve_on_small_lattices_stops(cuda_device):
+    """Zero sources, the iteration limit and sources that are not finite end the solve."""
+    from tfleonardym_b200 import _lib, dirac_solver
+    rng = np.random.default_rng(5)
+    geom, nc = (8, 12), 2
+    op = make_op(smooth_links(rng, geom, nc), geom, 0.12, True, "fundamental")
+    b = cnormal(rng, (3, 2, nc, 96))
+    b[1] = 0
+    for precision in ("f64", "f32", "f16"):
+        solver = dirac_solver.conjugate_gradient(max_steps=3, tol=1e-12, precision=precision)
+        x = solver.solve(op, cu(b)).cpu().numpy()
+        assert [r["iterations"] for r in solver.reports] == [3, 0, 3]
+        assert [r["status"] for r in solver.reports] == [_lib.LYM_ERR_NOT_CONVERGED, 0, _lib.LYM_ERR_NOT_CONVERGED]
+        assert np.all(x[1] == 0) and np.all(np.isfinite(x))
+        c = b.copy()
+        c[2, 0, 0, 5] = np.nan
+        solver = dirac_solver.conjugate_gradient(tol=1e-10, precision=precision)
+        x = solver.solve(op, cu(c)).cpu().numpy()
+        assert [r["status"] for r in solver.reports] == [0, 0, _lib.LYM_ERR_NOT_CONVERGED]
+        assert np.all(np.isfinite(x[:2]))
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32", "f16"])
+@pytest.mark.parametrize("geoms,nc", [([(8, 8), (4, 6), (32, 34), (2, 4)], 2),
+                                      ([(4, 4, 4, 4), (2, 4, 6, 8), (4, 4, 4, 10)], 3),
+                                      ([(4, 4, 4), (18, 16, 16), (8, 6, 4)], 2)])
+def test_lattices_of_uneven_sizes_together(cuda_device, geoms, nc, precision):
+    """Every lattice's own kappa, tolerance and number of sources; the last list has a lattice
+    above the resident form's limit, so it runs launch by launch."""
+    from tfleonardym_b200 import dirac_solver
+    rng = np.random.default_rng(len(geoms) + nc)
+    ops, bs, refs = [], [], []
+    for k, g in enumerate(geoms):
+        nd, vol = len(g), int(np.prod(g))
+        u = smooth_links(rng, g, nc)
+        kappa = 0.10 + 0.01 * k
+        ops.append(make_op(u, g, kappa, False, "fundamental"))
+        bs.append(cnormal(rng, (1 + k, 4 if nd == 4 else 2, nc, vol)))
+        refs.append((O.apply_time_bc(u, O.antiperiodic_field(g, BC)), kappa, O.lookup_tables(g)))
+    tols = [1e-10, 1e-9, 1e-11, 1e-10][:len(geoms)]
+    xs, reports = dirac_solver.solve_lattices(ops, [cu(b) for b in bs], precision=precision, tols=tols)
+    for k in range(len(geoms)):
+        for i in range(bs[k].shape[0]):
+            res = np.linalg.norm(bs[k][i] - O.wilson_apply(refs[k][0], xs[k][i].cpu().numpy(), refs[k][1], False,
+                                                           refs[k][2])) / np.linalg.norm(bs[k][i])
+            assert res < tols[k], (k, i, reports[k][i])
+            assert reports[k][i]["status"] == 0

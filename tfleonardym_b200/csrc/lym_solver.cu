@@ -28,6 +28,7 @@
 #include "lym_hop_tc.cuh"
 #include "lym_internal.cuh"
 #include "lym_kernels.cuh"
+#include "lym_small.cuh"
 
 namespace lym {
 
@@ -871,6 +872,11 @@ struct Work {
   cudaEvent_t ev_in = nullptr, ev_out = nullptr;
   cudaEvent_t ev_state[2] = {nullptr, nullptr};  // the two state copies in flight
   int64_t launches = 0;           // kernels launched by the current call (graph nodes included)
+  // descriptors and reports of the multi-lattice calls that this workspace leads: device
+  // memory with a pinned host copy, grown as needed
+  char* multi = nullptr;
+  char* multi_host = nullptr;
+  size_t multi_bytes = 0;
 };
 
 // Launch a kernel, or, while build_graph records, append it to the graph as a
@@ -1135,6 +1141,8 @@ static void free_work(Work* w) {
   if (w->st_host) cudaFreeHost(w->st_host);
   if (w->upd_host) cudaFreeHost(w->upd_host);
   if (w->res_host) cudaFreeHost(w->res_host);
+  if (w->multi) cudaFree(w->multi);
+  if (w->multi_host) cudaFreeHost(w->multi_host);
   delete w;
 }
 
@@ -1507,6 +1515,67 @@ static int autotune(Work& w, cudaStream_t st, int forced_rhs, int forced_comp, i
 static int cg_solve_on(Work& w, lym_gauge* g, double kappa, int nrhs, const void* b, void* x,
                        const lym_solver_params* prm, lym_solver_report* rep, cudaStream_t st);
 
+// The lattice of workspace w for the resident solver (lym_small.cu).
+static SmallLat small_lat(const Work& w, double kappa, const void* b, void* x, const lym_solver_params* prm, double tol,
+                          int sys0, SmallReport* rep) {
+  SmallLat L{};
+  L.g = w.g->geom;
+  L.hg64 = w.hg64;
+  L.hgs = w.hgs_f;
+  L.be = w.be;
+  L.bo = w.bo;
+  L.bp = w.bp;
+  L.x64 = w.x64;
+  L.s64 = w.s64;
+  L.r = w.r;
+  L.p = w.p;
+  L.t = w.t;
+  L.s = w.s;
+  L.xs = w.xs;
+  L.b = (const double2*)b;
+  L.x = (double2*)x;
+  L.kappa = kappa;
+  L.tol = tol;
+  L.delta = prm->delta > 0 && prm->delta < 1 ? prm->delta : 0.1;
+  L.hermitian = prm->hermitian ? 1 : 0;
+  L.max_iter = prm->max_iter;
+  L.nrhs = w.nreal;
+  L.sys0 = sys0;
+  L.rep = rep;
+  return L;
+}
+
+// Fills a call's reports from the device's; returns the status of the call.
+static int small_reports(const SmallReport* d, int n, int64_t launches, lym_solver_report* rep) {
+  int status = LYM_OK;
+  for (int i = 0; i < n; ++i) {
+    rep[i].status = d[i].done ? LYM_OK : LYM_ERR_NOT_CONVERGED;
+    rep[i].iterations = d[i].iterations;
+    rep[i].reliable_updates = d[i].updates;
+    rep[i].true_residual = d[i].true_residual;
+    rep[i].kernel_launches = launches;
+    rep[i].rhs_per_thread = 1;
+    rep[i].compressed_links = 0;
+    rep[i].mixed_fma = 0;
+    if (!d[i].done) status = LYM_ERR_NOT_CONVERGED;
+  }
+  return status;
+}
+
+static int cg_solve_small(Work& w, double kappa, int nrhs, const void* b, void* x, const lym_solver_params* prm,
+                          lym_solver_report* rep, cudaStream_t st) {
+  w.kappa = kappa;
+  w.dirty = std::max(w.dirty, w.nreal);
+  static_assert(sizeof(SmallReport) <= 8 * sizeof(double), "the workspace keeps eight result doubles per rhs");
+  SmallReport* d = reinterpret_cast<SmallReport*>(w.res);
+  const SmallLat one = small_lat(w, kappa, b, x, prm, prm->tol, 0, d);
+  const int rc = small_launch(w.g->nd, w.g->nc, w.sp, w.Vh, nullptr, 1, one, nrhs, st);
+  if (rc) return rc;
+  LYM_CUDA(cudaMemcpyAsync(w.res_host, d, sizeof(SmallReport) * nrhs, cudaMemcpyDeviceToHost, st));
+  LYM_CUDA(cudaStreamSynchronize(st));
+  return small_reports(reinterpret_cast<const SmallReport*>(w.res_host), nrhs, 1, rep);
+}
+
 static int cg_solve(lym_gauge* g, double kappa, int nrhs, const void* b, void* x, const lym_solver_params* prm,
                     lym_solver_report* rep, cudaStream_t caller) {
   LYM_REQUIRE(g && b && x && prm && rep, LYM_ERR_BAD_ARG, "null argument");
@@ -1526,7 +1595,10 @@ static int cg_solve(lym_gauge* g, double kappa, int nrhs, const void* b, void* x
   // order the solve after the caller's prior work, and the caller's later work after the solve
   LYM_CUDA(cudaEventRecord(w.ev_in, caller));
   LYM_CUDA(cudaStreamWaitEvent(w.stream, w.ev_in, 0));
-  rc = cg_solve_on(w, g, kappa, nrhs, b, x, prm, rep, w.stream);
+  if (prm->rhs_per_thread == 0 && small_applies(g->nd, g->nc, sp, g->Vh, nrhs, 1, prm->max_iter))
+    rc = cg_solve_small(w, kappa, nrhs, b, x, prm, rep, w.stream);
+  else
+    rc = cg_solve_on(w, g, kappa, nrhs, b, x, prm, rep, w.stream);
   cudaEventRecord(w.ev_out, w.stream);
   cudaStreamWaitEvent(caller, w.ev_out, 0);
   return rc;
@@ -1882,6 +1954,26 @@ static bool multi_pick(int nd, int nc, int sp, bool comp, MultiOps* out) {
   return true;
 }
 
+// At least `bytes` of w's multi-lattice buffer (a stream-ordered allocation per call was
+// returned to the system at every synchronisation and mapped again by the next call, a
+// millisecond or more).
+static int multi_buffer(Work& w, size_t bytes) {
+  if (w.multi_bytes >= bytes) return LYM_OK;
+  if (w.stream) LYM_CUDA(cudaStreamSynchronize(w.stream));
+  if (w.multi) cudaFree(w.multi);
+  if (w.multi_host) cudaFreeHost(w.multi_host);
+  w.multi = w.multi_host = nullptr;
+  w.multi_bytes = 0;
+  bytes = (bytes + 16383) & ~(size_t)16383;
+  if (cudaMalloc(&w.multi, bytes) != cudaSuccess || cudaMallocHost(&w.multi_host, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    set_error("multi-lattice descriptors of %zu bytes do not fit", bytes);
+    return LYM_ERR_OOM;
+  }
+  w.multi_bytes = bytes;
+  return LYM_OK;
+}
+
 // Per-lattice CG bookkeeping of the multi-lattice driver (the same decisions
 // as cg_solve_on's, for one workspace).
 struct MultiLat {
@@ -1942,9 +2034,16 @@ static int cg_solve_multi(int nlat, lym_gauge* const* gs, const double* kappas, 
   MultiOps ops;
   LYM_REQUIRE(multi_pick(nd, nc, sp, comp_all, &ops), LYM_ERR_UNSUPPORTED, "unsupported (nd=%d, N=%d)", nd, nc);
   std::vector<MultiLat> lats(nlat);
+  int64_t vh_max = 0;
+  int systems = 0;
   for (int l = 0; l < nlat; ++l) {
     int rc = get_work(gs[l], nrhs[l], sp, &lats[l].w);
     if (rc) return rc;
+    vh_max = std::max(vh_max, gs[l]->Vh);
+    systems += nrhs[l];
+  }
+  const bool small = prm->rhs_per_thread == 0 && small_applies(nd, nc, sp, vh_max, systems, nlat, prm->max_iter);
+  for (int l = 0; l < nlat && !small; ++l) {
     Work& w = *lats[l].w;
     int pick = -1;
     for (int i = 0; i < w.ncand; ++i)
@@ -1963,6 +2062,27 @@ static int cg_solve_multi(int nlat, lym_gauge* const* gs, const double* kappas, 
       cudaStreamWaitEvent(to, ev, 0);
     }
   } fence{lats[0].w->ev_out, st, caller};
+  if (small) {
+    // one launch for every right-hand side of every lattice, one copy back
+    Work& lead = *lats[0].w;
+    const size_t dbytes = (sizeof(SmallLat) * nlat + 255) & ~(size_t)255, rbytes = sizeof(SmallReport) * systems;
+    int rc = multi_buffer(lead, dbytes + rbytes);
+    if (rc) return rc;
+    SmallLat* desc = reinterpret_cast<SmallLat*>(lead.multi_host);
+    SmallReport* drep = reinterpret_cast<SmallReport*>(lead.multi + dbytes);
+    for (int l = 0, s0 = 0; l < nlat; s0 += nrhs[l], ++l) {
+      Work& w = *lats[l].w;
+      w.kappa = kappas[l];
+      w.dirty = std::max(w.dirty, w.nreal);
+      desc[l] = small_lat(w, kappas[l], bs[l], xs[l], prm, tols ? tols[l] : prm->tol, s0, drep + s0);
+    }
+    LYM_CUDA(cudaMemcpyAsync(lead.multi, desc, sizeof(SmallLat) * nlat, cudaMemcpyHostToDevice, st));
+    rc = small_launch(nd, nc, sp, vh_max, reinterpret_cast<SmallLat*>(lead.multi), nlat, desc[0], systems, st);
+    if (rc) return rc;
+    LYM_CUDA(cudaMemcpyAsync(lead.multi_host + dbytes, drep, rbytes, cudaMemcpyDeviceToHost, st));
+    LYM_CUDA(cudaStreamSynchronize(st));
+    return small_reports(reinterpret_cast<const SmallReport*>(lead.multi_host + dbytes), systems, 1, rep);
+  }
   const double delta = prm->delta > 0 && prm->delta < 1 ? prm->delta : 0.1;
   const int chunk = prm->chunk > 0 ? std::min(prm->chunk, 256) : 8;
   EoField none;
@@ -1998,18 +2118,17 @@ static int cg_solve_multi(int nlat, lym_gauge* const* gs, const double* kappas, 
                 "too many blocks for one launch");
     blocks += w.nblk * w.nrhs;
   }
-  CgLat* d_desc = nullptr;
-  LYM_CUDA(cudaMallocAsync(&d_desc, sizeof(CgLat) * nlat, st));
+  int rcb = multi_buffer(*lats[0].w, sizeof(CgLat) * nlat);
+  if (rcb) return rcb;
+  CgLat* d_desc = reinterpret_cast<CgLat*>(lats[0].w->multi);
   struct Release {
-    CgLat* p;
-    cudaStream_t st;
     cudaGraphExec_t exec = nullptr;
     ~Release() {
       if (exec) cudaGraphExecDestroy(exec);
-      cudaFreeAsync(p, st);
     }
-  } release{d_desc, st};
-  LYM_CUDA(cudaMemcpyAsync(d_desc, desc.data(), sizeof(CgLat) * nlat, cudaMemcpyHostToDevice, st));
+  } release;
+  std::memcpy(lats[0].w->multi_host, desc.data(), sizeof(CgLat) * nlat);
+  LYM_CUDA(cudaMemcpyAsync(d_desc, lats[0].w->multi_host, sizeof(CgLat) * nlat, cudaMemcpyHostToDevice, st));
   int64_t launches = 0;
   // FP64 reliable update of every lattice's rhs with upd set, in launches over all
   // lattices; |q|^2 lands in res_host[0..n), |r|^2 in res_host[n..2n)
