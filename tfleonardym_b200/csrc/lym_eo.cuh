@@ -236,6 +236,7 @@ struct EoGeom {
   // with bit 31 set when the hop crosses the time boundary (mu = nd-1 and the
   // link involved sits on the last time slice).  Built once per gauge object.
   const int* nbr;
+  int tile_fast;  // hop kernels of lym_solver.cu: grid (rhs tiles, site blocks), else (site blocks, rhs tiles)
 };
 constexpr int kNbrBoundary = int(0x80000000u);
 

@@ -282,6 +282,32 @@ __global__ void zero64_kernel(int64_t Vh, EoField f) {
   store_sp<SP64, NCOMP>(f, blockIdx.y, cb, z);
 }
 
+// The hop kernels' block of sites bx and rhs tile by.  Two orders of the grid: with the tile
+// as the slow index each tile walks the whole lattice, its spinors staying in L2; with the
+// tile fastest (EoGeom::tile_fast) the blocks that read one site block's links run back to
+// back and all but the first find them in L2.  See HopGrid.
+LYM_D void rhs_tile(const EoGeom& g, int& bx, int& by) {
+  bx = (int)(g.tile_fast ? blockIdx.y : blockIdx.x);
+  by = (int)(g.tile_fast ? blockIdx.x : blockIdx.y);
+}
+
+// Grid for nblk site blocks x tiles over links of `link_bytes`: the tile fastest where the
+// links do not stay in L2 between two walks of the lattice (half of the 126 MB, the rest
+// being the spinors').  24^3 x 48 SU(3): FP64 hop (382 MB of links), 4 rhs, 245 us against
+// 299 us, the solve 115 against 137 ms; FP16 (106 MB), 8 rhs, the solve 93.6 against
+// 98.5 ms.  16^4 (FP64 38 MB, 12 rhs): 66 us against 57 us the other way, FP16 16 rhs 20.2
+// against 17.6 us, so the slow tile stays below.
+struct HopGrid {
+  EoGeom g;
+  dim3 grid;
+  HopGrid(const EoGeom& geom, int nblk, int tiles, size_t link_bytes) : g(geom), grid(nblk, tiles) {
+    if (tiles > 1 && nblk <= 65535 && link_bytes > (size_t)64 << 20) {
+      g.tile_fast = 1;
+      grid = dim3(tiles, nblk);
+    }
+  }
+};
+
 // ---------------------------------------------------------------------------
 // FP64 hop with a linear-combination epilogue (reliable updates, setup):
 //   out = z0 + a1 z1 + c * G5OUT(hop(G5IN(in)))  ; optional |out|^2 -> res[rhs]
@@ -329,8 +355,10 @@ __global__ void __launch_bounds__(128, 1) hop64_lincomb_kernel(EoGeom g, HopGaug
                                                             EoField z0, EoField z1, double a1, double c,
                                                             const int* upd, double* partials, unsigned* counters,
                                                             double* res, int nblk) {
-  hop64_lincomb_body<ND, NC, G5IN, G5OUT>(g, hg, in, par, out, z0, z1, a1, c, upd, partials, counters, res, nblk,
-                                          blockIdx.x, blockIdx.y);
+  int bx, by;
+  rhs_tile(g, bx, by);
+  hop64_lincomb_body<ND, NC, G5IN, G5OUT>(g, hg, in, par, out, z0, z1, a1, c, upd, partials, counters, res, nblk, bx,
+                                          by);
 }
 
 // |f|^2 per rhs (FP64 field)
@@ -398,7 +426,9 @@ LYM_D void cg_hop_body(const EoGeom& g, const HopGauge& hg, const EoField& in, c
 template <int ND, int NC, int SP, int GP, bool COMP, bool G5IN, int R, int MX>
 __global__ void __launch_bounds__(128, SP == SP64 ? 1 : 0) cg_hop_kernel(EoGeom g, HopGauge hg, EoField in, EoField out, int par,
                                                      const CGState* st) {
-  cg_hop_body<ND, NC, SP, GP, COMP, G5IN, R, MX>(g, hg, in, out, par, st, blockIdx.x, blockIdx.y);
+  int bx, by;
+  rhs_tile(g, bx, by);
+  cg_hop_body<ND, NC, SP, GP, COMP, G5IN, R, MX>(g, hg, in, out, par, st, bx, by);
 }
 
 // t = p - kappa^2 H_eo s ; alpha = rr / |t|^2   (rhs tile of R)
@@ -459,7 +489,9 @@ LYM_D void cg_t_body(const EoGeom& g, const HopGauge& hg, const EoField& s, cons
 template <int ND, int NC, int SP, int GP, bool COMP, int R, int MX>
 __global__ void __launch_bounds__(128, SP == SP64 ? 1 : 0) cg_t_kernel(EoGeom g, HopGauge hg, EoField s, EoField p, EoField t, double k2,
                                                    CGState* st, double* partials, unsigned* counters, int nblk) {
-  cg_t_body<ND, NC, SP, GP, COMP, R, MX>(g, hg, s, p, t, k2, st, partials, counters, nblk, blockIdx.x, blockIdx.y);
+  int bx, by;
+  rhs_tile(g, bx, by);
+  cg_t_body<ND, NC, SP, GP, COMP, R, MX>(g, hg, s, p, t, k2, st, partials, counters, nblk, bx, by);
 }
 
 // Ap = t - kappa^2 gamma_d H_eo s ; r -= alpha Ap ; beta = |r|^2 / rr   (rhs tile of R).
@@ -529,8 +561,9 @@ __global__ void __launch_bounds__(128, SP == SP64 ? 1 : 0) cg_update_kernel(EoGe
                                                                            EoField r, double k2, CGState* st,
                                                                            double* partials, unsigned* counters,
                                                                            int nblk) {
-  cg_update_body<ND, NC, SP, GP, COMP, R, MX>(g, hg, s, t, r, k2, st, partials, counters, nblk, blockIdx.x,
-                                              blockIdx.y);
+  int bx, by;
+  rhs_tile(g, bx, by);
+  cg_update_body<ND, NC, SP, GP, COMP, R, MX>(g, hg, s, t, r, k2, st, partials, counters, nblk, bx, by);
 }
 
 // Reliable-update residual in the sloppy precision: r = t - kappa^2 gamma_d H_eo s
@@ -589,8 +622,9 @@ template <int ND, int NC, int SP, int GP, bool COMP, int R, int MX>
 __global__ void __launch_bounds__(128, SP == SP64 ? 1 : 0) cg_rnew_kernel(EoGeom g, HopGauge hg, EoField s, EoField t, EoField r,
                                                       double k2, const int* upd, double* partials,
                                                       unsigned* counters, double* res, int nblk) {
-  cg_rnew_body<ND, NC, SP, GP, COMP, R, MX>(g, hg, s, t, r, k2, upd, partials, counters, res, nblk, blockIdx.x,
-                                            blockIdx.y);
+  int bx, by;
+  rhs_tile(g, bx, by);
+  cg_rnew_body<ND, NC, SP, GP, COMP, R, MX>(g, hg, s, t, r, k2, upd, partials, counters, res, nblk, bx, by);
 }
 
 // dst = src (same precision) for rhs with upd[rhs]
@@ -901,28 +935,36 @@ struct Impl {
   // frequent reliable updates) and in the sloppy precision otherwise
   static constexpr int XP = (SP == SP16 || SP == SPB16) ? SP32 : SP;
 
+  // FP32 with one rhs per thread keeps the slow tile: with the tile fastest its bare hop, which
+  // the autotuner times, ties with the four-rhs form, whose iterations are 5 % faster
+  static HopGrid hop_tiles(const Work& w) {
+    const size_t link = SP == SP64 ? NC * NC * 16 : (size_t)w.hgs.nunits * (SP == SP32 ? 16 : 8);
+    return HopGrid(w.g->geom, w.nblk, w.nrhs / R, SP == SP32 && R == 1 ? 0 : w.g->V * w.g->nd * link);
+  }
+
   static void iterate(Work& w, cudaStream_t st) {
     const double k2 = w.kappa * w.kappa;
-    dim3 grid(w.nblk, w.nrhs), tile(w.nblk, w.nrhs / R);
+    const dim3 grid(w.nblk, w.nrhs);
+    const HopGrid h = hop_tiles(w);
     const CGState* cst = w.st;
-    launch(w, st, cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX>, tile, dim3(128), w.g->geom, w.hgs, w.p, w.s, 1,
+    launch(w, st, cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX>, h.grid, dim3(128), h.g, w.hgs, w.p, w.s, 1,
            cst);
-    launch(w, st, cg_t_kernel<ND, NC, SP, GP, COMP, R, MX>, tile, dim3(128), w.g->geom, w.hgs, w.s, w.p, w.t, k2,
+    launch(w, st, cg_t_kernel<ND, NC, SP, GP, COMP, R, MX>, h.grid, dim3(128), h.g, w.hgs, w.s, w.p, w.t, k2,
            w.st, w.partials, w.counters, w.nblk);
-    launch(w, st, cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX>, tile, dim3(128), w.g->geom, w.hgs, w.t, w.s, 1,
+    launch(w, st, cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX>, h.grid, dim3(128), h.g, w.hgs, w.t, w.s, 1,
            cst);
-    launch(w, st, cg_update_kernel<ND, NC, SP, GP, COMP, R, MX>, tile, dim3(128), w.g->geom, w.hgs, w.s, w.t, w.r,
+    launch(w, st, cg_update_kernel<ND, NC, SP, GP, COMP, R, MX>, h.grid, dim3(128), h.g, w.hgs, w.s, w.t, w.r,
            k2, w.st, w.partials, w.counters, w.nblk);
     launch(w, st, cg_p_kernel<SP, XP, NCOMP>, grid, dim3(128), w.Vh, w.r, w.p, w.xs, w.st, w.counters);
   }
 
   static void hop64(Work& w, int par, const EoField& in, const EoField& out, const EoField& z0, const EoField& z1,
                     double a1, double c, bool g5in, bool g5out, bool with_norm, cudaStream_t st) {
-    dim3 grid(w.nblk, w.nrhs);
+    const HopGrid h(w.g->geom, w.nblk, w.nrhs, w.g->V * w.g->nd * (size_t)(NC * NC * 16));
     double* res = with_norm ? w.res : nullptr;
     w.launches += 1;
 #define LYM_H64(A, B)                                                                                   \
-  hop64_lincomb_kernel<ND, NC, A, B><<<grid, 128, 0, st>>>(w.g->geom, w.hg64, in, par, out, z0, z1, a1, c, \
+  hop64_lincomb_kernel<ND, NC, A, B><<<h.grid, 128, 0, st>>>(h.g, w.hg64, in, par, out, z0, z1, a1, c, \
                                                            w.upd, w.partials, w.counters, res, w.nblk)
     if (g5in && g5out) LYM_H64(true, true);
     else if (g5in) LYM_H64(true, false);
@@ -965,16 +1007,16 @@ struct Impl {
     zero64_kernel<NCOMP><<<grid, 128, 0, st>>>(w.Vh, f);
   }
   static void dslash(Work& w, cudaStream_t st) {
-    dim3 tile(w.nblk, w.nrhs / R);
+    const HopGrid h = hop_tiles(w);
     w.launches += 1;
-    cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX><<<tile, 128, 0, st>>>(w.g->geom, w.hgs, w.p, w.s, 1, nullptr);
+    cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX><<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.p, w.s, 1, nullptr);
   }
   static void rnew(Work& w, cudaStream_t st) {
     const double k2 = w.kappa * w.kappa;
-    dim3 tile(w.nblk, w.nrhs / R);
+    const HopGrid h = hop_tiles(w);
     w.launches += 2;
-    cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX><<<tile, 128, 0, st>>>(w.g->geom, w.hgs, w.t, w.s, 1, nullptr);
-    cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX><<<tile, 128, 0, st>>>(w.g->geom, w.hgs, w.s, w.t, w.r, k2, w.upd,
+    cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX><<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.t, w.s, 1, nullptr);
+    cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX><<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.s, w.t, w.r, k2, w.upd,
                                                                       w.partials, w.counters, w.res, w.nblk);
   }
   static void copy_rp(Work& w, cudaStream_t st) {
