@@ -297,9 +297,12 @@ LYM_D void rhs_tile(const EoGeom& g, int& bx, int& by) {
 // 299 us, the solve 115 against 137 ms; FP16 (106 MB), 8 rhs, the solve 93.6 against
 // 98.5 ms.  16^4 (FP64 38 MB, 12 rhs): 66 us against 57 us the other way, FP16 16 rhs 20.2
 // against 17.6 us, so the slow tile stays below.
+constexpr unsigned kDenseFrom = 2 * 2 * 148;  // blocks: two waves of two per SM
+
 struct HopGrid {
   EoGeom g;
   dim3 grid;
+  bool dense() const { return grid.x * grid.y > kDenseFrom; }  // FP64 hop kernels: three blocks per SM
   HopGrid(const EoGeom& geom, int nblk, int tiles, size_t link_bytes) : g(geom), grid(nblk, tiles) {
     if (tiles > 1 && nblk <= 65535 && link_bytes > (size_t)64 << 20) {
       g.tile_fast = 1;
@@ -350,8 +353,8 @@ LYM_D void hop64_lincomb_body(const EoGeom& g, const HopGauge& hg, const EoField
   }
 }
 
-template <int ND, int NC, bool G5IN, bool G5OUT>
-__global__ void __launch_bounds__(128, 1) hop64_lincomb_kernel(EoGeom g, HopGauge hg, EoField in, int par, EoField out,
+template <int ND, int NC, bool G5IN, bool G5OUT, int MINB = 1>
+__global__ void __launch_bounds__(128, MINB) hop64_lincomb_kernel(EoGeom g, HopGauge hg, EoField in, int par, EoField out,
                                                             EoField z0, EoField z1, double a1, double c,
                                                             const int* upd, double* partials, unsigned* counters,
                                                             double* res, int nblk) {
@@ -385,8 +388,13 @@ __global__ void __launch_bounds__(128) norm64_kernel(int64_t Vh, EoField f, doub
 
 // Launch bounds of the hop kernels: FP64 ones declare one resident block per
 // SM as enough, which lets ptxas keep every neighbour's loads in flight at once
-// (about 250 registers); the memory-bound FP64 hop runs ~20% faster at 32^4
-// that way.  Sloppy ones keep ptxas's default register target.
+// (about 250 registers, two blocks); the memory-bound FP64 hop runs ~20% faster at
+// 32^4 than with ptxas's default register target.  Beyond two full waves of blocks
+// (kDenseFrom) a form with three blocks per SM (168 registers, a few spilled) is the
+// faster one: 24^3 x 48, the FP64 solve 109 against 115 ms with 4 rhs and 36.5 against
+// 37.3 ms with one, the FP16 one (its FP64 updates) 90.2 against 93.4 ms with 8; at 16^4
+// with one rhs (256 blocks) it is 1.5 % slower.  Sloppy kernels keep ptxas's default
+// register target.
 //
 // The kernel bodies below take the block's site block `bx` and rhs tile `by`
 // (and, for the reductions, the site-block count nblk) so that the
@@ -423,8 +431,8 @@ LYM_D void cg_hop_body(const EoGeom& g, const HopGauge& hg, const EoField& in, c
   }
 }
 
-template <int ND, int NC, int SP, int GP, bool COMP, bool G5IN, int R, int MX>
-__global__ void __launch_bounds__(128, SP == SP64 ? 1 : 0) cg_hop_kernel(EoGeom g, HopGauge hg, EoField in, EoField out, int par,
+template <int ND, int NC, int SP, int GP, bool COMP, bool G5IN, int R, int MX, int MINB = SP == SP64 ? 1 : 0>
+__global__ void __launch_bounds__(128, MINB) cg_hop_kernel(EoGeom g, HopGauge hg, EoField in, EoField out, int par,
                                                      const CGState* st) {
   int bx, by;
   rhs_tile(g, bx, by);
@@ -486,8 +494,8 @@ LYM_D void cg_t_body(const EoGeom& g, const HopGauge& hg, const EoField& s, cons
   }
 }
 
-template <int ND, int NC, int SP, int GP, bool COMP, int R, int MX>
-__global__ void __launch_bounds__(128, SP == SP64 ? 1 : 0) cg_t_kernel(EoGeom g, HopGauge hg, EoField s, EoField p, EoField t, double k2,
+template <int ND, int NC, int SP, int GP, bool COMP, int R, int MX, int MINB = SP == SP64 ? 1 : 0>
+__global__ void __launch_bounds__(128, MINB) cg_t_kernel(EoGeom g, HopGauge hg, EoField s, EoField p, EoField t, double k2,
                                                    CGState* st, double* partials, unsigned* counters, int nblk) {
   int bx, by;
   rhs_tile(g, bx, by);
@@ -556,8 +564,8 @@ LYM_D void cg_update_body(const EoGeom& g, const HopGauge& hg, const EoField& s,
   }
 }
 
-template <int ND, int NC, int SP, int GP, bool COMP, int R, int MX>
-__global__ void __launch_bounds__(128, SP == SP64 ? 1 : 0) cg_update_kernel(EoGeom g, HopGauge hg, EoField s, EoField t,
+template <int ND, int NC, int SP, int GP, bool COMP, int R, int MX, int MINB = SP == SP64 ? 1 : 0>
+__global__ void __launch_bounds__(128, MINB) cg_update_kernel(EoGeom g, HopGauge hg, EoField s, EoField t,
                                                                            EoField r, double k2, CGState* st,
                                                                            double* partials, unsigned* counters,
                                                                            int nblk) {
@@ -618,8 +626,8 @@ LYM_D void cg_rnew_body(const EoGeom& g, const HopGauge& hg, const EoField& s, c
   }
 }
 
-template <int ND, int NC, int SP, int GP, bool COMP, int R, int MX>
-__global__ void __launch_bounds__(128, SP == SP64 ? 1 : 0) cg_rnew_kernel(EoGeom g, HopGauge hg, EoField s, EoField t, EoField r,
+template <int ND, int NC, int SP, int GP, bool COMP, int R, int MX, int MINB = SP == SP64 ? 1 : 0>
+__global__ void __launch_bounds__(128, MINB) cg_rnew_kernel(EoGeom g, HopGauge hg, EoField s, EoField t, EoField r,
                                                       double k2, const int* upd, double* partials,
                                                       unsigned* counters, double* res, int nblk) {
   int bx, by;
@@ -934,6 +942,7 @@ struct Impl {
   // norm-scaled half accumulator loses the small late corrections and forces
   // frequent reliable updates) and in the sloppy precision otherwise
   static constexpr int XP = (SP == SP16 || SP == SPB16) ? SP32 : SP;
+  static constexpr int MB = SP == SP64 ? 1 : 0, DB = SP == SP64 ? 3 : 0;  // blocks per SM declared: usual, dense form
 
   // FP32 with one rhs per thread keeps the slow tile: with the tile fastest its bare hop, which
   // the autotuner times, ties with the four-rhs form, whose iterations are 5 % faster
@@ -947,15 +956,21 @@ struct Impl {
     const dim3 grid(w.nblk, w.nrhs);
     const HopGrid h = hop_tiles(w);
     const CGState* cst = w.st;
-    launch(w, st, cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX>, h.grid, dim3(128), h.g, w.hgs, w.p, w.s, 1,
-           cst);
-    launch(w, st, cg_t_kernel<ND, NC, SP, GP, COMP, R, MX>, h.grid, dim3(128), h.g, w.hgs, w.s, w.p, w.t, k2,
-           w.st, w.partials, w.counters, w.nblk);
-    launch(w, st, cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX>, h.grid, dim3(128), h.g, w.hgs, w.t, w.s, 1,
-           cst);
-    launch(w, st, cg_update_kernel<ND, NC, SP, GP, COMP, R, MX>, h.grid, dim3(128), h.g, w.hgs, w.s, w.t, w.r,
-           k2, w.st, w.partials, w.counters, w.nblk);
+    if (h.dense()) iterate_hops<DB>(w, st, h, cst, k2);
+    else iterate_hops<MB>(w, st, h, cst, k2);
     launch(w, st, cg_p_kernel<SP, XP, NCOMP>, grid, dim3(128), w.Vh, w.r, w.p, w.xs, w.st, w.counters);
+  }
+
+  template <int M>
+  static void iterate_hops(Work& w, cudaStream_t st, const HopGrid& h, const CGState* cst, double k2) {
+    launch(w, st, cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX, M>, h.grid, dim3(128), h.g, w.hgs, w.p, w.s, 1,
+           cst);
+    launch(w, st, cg_t_kernel<ND, NC, SP, GP, COMP, R, MX, M>, h.grid, dim3(128), h.g, w.hgs, w.s, w.p, w.t, k2,
+           w.st, w.partials, w.counters, w.nblk);
+    launch(w, st, cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX, M>, h.grid, dim3(128), h.g, w.hgs, w.t, w.s, 1,
+           cst);
+    launch(w, st, cg_update_kernel<ND, NC, SP, GP, COMP, R, MX, M>, h.grid, dim3(128), h.g, w.hgs, w.s, w.t, w.r,
+           k2, w.st, w.partials, w.counters, w.nblk);
   }
 
   static void hop64(Work& w, int par, const EoField& in, const EoField& out, const EoField& z0, const EoField& z1,
@@ -963,9 +978,11 @@ struct Impl {
     const HopGrid h(w.g->geom, w.nblk, w.nrhs, w.g->V * w.g->nd * (size_t)(NC * NC * 16));
     double* res = with_norm ? w.res : nullptr;
     w.launches += 1;
-#define LYM_H64(A, B)                                                                                   \
-  hop64_lincomb_kernel<ND, NC, A, B><<<h.grid, 128, 0, st>>>(h.g, w.hg64, in, par, out, z0, z1, a1, c, \
-                                                           w.upd, w.partials, w.counters, res, w.nblk)
+    auto run = [&](auto kernel) {
+      kernel<<<h.grid, 128, 0, st>>>(h.g, w.hg64, in, par, out, z0, z1, a1, c, w.upd, w.partials, w.counters, res,
+                                     w.nblk);
+    };
+#define LYM_H64(A, B) run(h.dense() ? hop64_lincomb_kernel<ND, NC, A, B, 3> : hop64_lincomb_kernel<ND, NC, A, B, 1>)
     if (g5in && g5out) LYM_H64(true, true);
     else if (g5in) LYM_H64(true, false);
     else if (g5out) LYM_H64(false, true);
@@ -1009,14 +1026,19 @@ struct Impl {
   static void dslash(Work& w, cudaStream_t st) {
     const HopGrid h = hop_tiles(w);
     w.launches += 1;
-    cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX><<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.p, w.s, 1, nullptr);
+    auto hop = h.dense() ? cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX, DB>
+                         : cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX, MB>;
+    hop<<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.p, w.s, 1, nullptr);
   }
   static void rnew(Work& w, cudaStream_t st) {
     const double k2 = w.kappa * w.kappa;
     const HopGrid h = hop_tiles(w);
     w.launches += 2;
-    cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX><<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.t, w.s, 1, nullptr);
-    cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX><<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.s, w.t, w.r, k2, w.upd,
+    auto hop = h.dense() ? cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX, DB>
+                         : cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX, MB>;
+    auto rnew = h.dense() ? cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX, DB> : cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX, MB>;
+    hop<<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.t, w.s, 1, nullptr);
+    rnew<<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.s, w.t, w.r, k2, w.upd,
                                                                       w.partials, w.counters, w.res, w.nblk);
   }
   static void copy_rp(Work& w, cudaStream_t st) {
@@ -1032,6 +1054,12 @@ struct Impl {
     cudaFuncGetAttributes(&a, cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX>);
     cudaFuncGetAttributes(&a, cg_t_kernel<ND, NC, SP, GP, COMP, R, MX>);
     cudaFuncGetAttributes(&a, cg_update_kernel<ND, NC, SP, GP, COMP, R, MX>);
+    if constexpr (DB != MB) {
+      cudaFuncGetAttributes(&a, cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX, DB>);
+      cudaFuncGetAttributes(&a, cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX, DB>);
+      cudaFuncGetAttributes(&a, cg_t_kernel<ND, NC, SP, GP, COMP, R, MX, DB>);
+      cudaFuncGetAttributes(&a, cg_update_kernel<ND, NC, SP, GP, COMP, R, MX, DB>);
+    }
     cudaFuncGetAttributes(&a, cg_p_kernel<SP, XP, NCOMP>);
   }
 
