@@ -120,8 +120,8 @@ LYM_D int eo_block_parity(int nblk) { return blockIdx.x >= (unsigned)nblk ? 1 : 
 // ---------------------------------------------------------------------------
 
 // w = p + kappa H p (p = the base direction); |w|^2 and |p|^2 -> alpha
-template <int ND, int NC, int SP, int GP, bool COMP, int R, int MX>
-__global__ void __launch_bounds__(128, SP == SP64 ? 1 : 0)
+template <int ND, int NC, int SP, int GP, bool COMP, int R, int MX, int MINB = SP == SP64 ? 1 : 0>
+__global__ void __launch_bounds__(128, MINB)
     ms_dp_kernel(EoGeom g, HopGauge hg, EoField pb, EoField w, int G, double kappa, MsGroup* grp,
                  double* partials, unsigned* counters, int nblk) {
   constexpr int NS = Gamma<ND>::NS, NCOMP = NS * NC;
@@ -182,8 +182,8 @@ __global__ void __launch_bounds__(128, SP == SP64 ? 1 : 0)
 
 // r -= alpha (w + kappa gamma_d H gamma_d w + sigma_0 p); |r|^2 -> beta; the
 // last block then advances every shift's recurrences (one thread per shift)
-template <int ND, int NC, int SP, int GP, bool COMP, int R, int MX>
-__global__ void __launch_bounds__(128, SP == SP64 ? 1 : 0)
+template <int ND, int NC, int SP, int GP, bool COMP, int R, int MX, int MINB = SP == SP64 ? 1 : 0>
+__global__ void __launch_bounds__(128, MINB)
     ms_ap_kernel(EoGeom g, HopGauge hg, EoField w, EoField pb, EoField ring, int G, int S, double kappa,
                  MsGroup* grp, MsShift* shf, double* partials, unsigned* counters, int nblk) {
   constexpr int NS = Gamma<ND>::NS, NCOMP = NS * NC;
@@ -746,10 +746,27 @@ struct MsImpl {
 
   static void iterate(MsWork& w, cudaStream_t st, int i) {
     dim3 tile(2 * w.nblk, w.G / R), grid(2 * w.nblk, w.G);
-    ms_launch(w, st, ms_dp_kernel<ND, NC, SP, GP, COMP, R, MX>, tile, dim3(128), w.g->geom, w.hgs, w.pb, w.w, w.G,
-              w.kappa, w.grp, w.partials, w.counters + w.G, w.nblk);
-    ms_launch(w, st, ms_ap_kernel<ND, NC, SP, GP, COMP, R, MX>, tile, dim3(128), w.g->geom, w.hgs, w.w, w.pb, w.ring,
-              w.G, w.S, w.kappa, w.grp, w.shf, w.partials, w.counters + w.G, w.nblk);
+    // FP64 kernels hold about 250 registers, two blocks per SM; where that leaves a last wave
+    // nearly empty, the form with three blocks per SM (168 registers, a few spilled) runs
+    // fewer waves of about 1.2 times the length.  12^3 x 24, one source (324 blocks, two
+    // waves or one): 12.8 and 15.4 us against 16.6 and 19.0 us, the solve 8.5 against 9.8 ms;
+    // at one wave of each (8^3 x 16) or several (16^4, 24^3 x 48) it is 2 to 13 % slower.
+    bool dense = false;
+    if constexpr (SP == SP64) {
+      const int n = 2 * w.nblk * (w.G / R), w2 = (n + 295) / 296, w3 = (n + 443) / 444;
+      dense = w2 <= 3 && 5 * w2 > 6 * w3;
+    }
+    auto run = [&](auto dp, auto ap) {
+      ms_launch(w, st, dp, tile, dim3(128), w.g->geom, w.hgs, w.pb, w.w, w.G, w.kappa, w.grp, w.partials,
+                w.counters + w.G, w.nblk);
+      ms_launch(w, st, ap, tile, dim3(128), w.g->geom, w.hgs, w.w, w.pb, w.ring, w.G, w.S, w.kappa, w.grp, w.shf,
+                w.partials, w.counters + w.G, w.nblk);
+    };
+    constexpr int kDense = SP == SP64 ? 3 : 0;
+    if (dense)
+      run(ms_dp_kernel<ND, NC, SP, GP, COMP, R, MX, kDense>, ms_ap_kernel<ND, NC, SP, GP, COMP, R, MX, kDense>);
+    else
+      run(ms_dp_kernel<ND, NC, SP, GP, COMP, R, MX>, ms_ap_kernel<ND, NC, SP, GP, COMP, R, MX>);
     ms_launch(w, st, ms_p0_kernel<SP, XP, NCOMP>, grid, dim3(128), w.Vh, w.nblk, w.G, w.S, w.ring, w.pb, w.xs, w.grp,
               w.counters);
     if ((i + 1) % kMsBlock == 0) {
@@ -803,6 +820,10 @@ struct MsImpl {
     cudaFuncAttributes a;
     cudaFuncGetAttributes(&a, ms_dp_kernel<ND, NC, SP, GP, COMP, R, MX>);
     cudaFuncGetAttributes(&a, ms_ap_kernel<ND, NC, SP, GP, COMP, R, MX>);
+    if constexpr (SP == SP64) {
+      cudaFuncGetAttributes(&a, ms_dp_kernel<ND, NC, SP, GP, COMP, R, MX, 3>);
+      cudaFuncGetAttributes(&a, ms_ap_kernel<ND, NC, SP, GP, COMP, R, MX, 3>);
+    }
     cudaFuncGetAttributes(&a, ms_p0_kernel<SP, XP, NCOMP>);
     if constexpr (SP == SP64 || SP == SP32) {
       constexpr int NU = units_for(NCOMP, Prec<SP>::CPU);
