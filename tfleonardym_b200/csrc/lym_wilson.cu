@@ -113,10 +113,16 @@ LYM_D void full_hop(int mu, int s, const cx<double> (&u)[NC][NC], const double2*
 // group fastest (block b: group b % ngroups, site block b / ngroups), so the blocks
 // that read one site block's links run back to back and all but the first find the
 // links in L2: each link crosses HBM about once per launch, not once per vector.
-// One resident block per SM is declared enough, so ptxas keeps every neighbour's
-// loads in flight at once (memory-bound FP64 stencil).
-template <int ND, int NC, bool HERM, int R>
-__global__ void __launch_bounds__(128, 1) wilson_full_kernel(
+// Bound by the latency of the neighbour gathers (FP64 pipe 25 %, L1 42 %, no memory level
+// above 60 % of its rate), so warps count as long as nothing much spills: in four
+// dimensions 12 warps per SM (168 registers) in blocks of two, one vector per thread.
+// 32^4 SU(3), one vector: 214 us against 233 us with 8 warps (254 registers), 240 us with
+// 16 (spills); 12 vectors on 16^3 x 32: 267 us against 294 us for two vectors per thread
+// at 8 warps, which saves a quarter of the link loads.
+// Launches of one or two waves of 8 warps per SM stay with 254 registers, except where 12
+// warps need one wave and 8 need two: 16^4 SU(3), one vector, 14.4 against 15.7 us.
+template <int ND, int NC, bool HERM, int R, int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) wilson_full_kernel(
     const int32_t* __restrict__ tab, int V, int Lt, double kappa, double bcr, double bci,
     const double2* __restrict__ U, const double2* __restrict__ in, double2* __restrict__ out, int ngroups) {
   constexpr int NS = Gamma<ND>::NS;
@@ -173,30 +179,39 @@ __global__ void __launch_bounds__(128, 1) wilson_full_kernel(
   }
 }
 
+template <int ND, int NC, int R, int THREADS, int MINB>
+static void launch_form(const lym_lattice* lat, double kappa, int herm, double bcr, double bci, const void* gauge,
+                        int ngroups, const void* in, void* out, cudaStream_t st) {
+  const unsigned grid = grid_for(lat->V, THREADS) * (unsigned)ngroups;
+  const int Lt = lat->dims[ND - 1];
+  auto run = [&](auto kernel) {
+    kernel<<<grid, THREADS, 0, st>>>(lat->d_tab, (int)lat->V, Lt, kappa, bcr, bci, (const double2*)gauge,
+                                     (const double2*)in, (double2*)out, ngroups);
+  };
+  if constexpr (ND != 3) {  // no hermitian form in three dimensions
+    if (herm) return run(wilson_full_kernel<ND, NC, true, R, THREADS, MINB>);
+  }
+  run(wilson_full_kernel<ND, NC, false, R, THREADS, MINB>);
+}
+
 template <int ND, int NC, int R>
 static void launch_full_r(const lym_lattice* lat, double kappa, int herm, double bcr, double bci, const void* gauge,
                           int ngroups, const void* in, void* out, cudaStream_t st) {
-  const unsigned grid = grid_for(lat->V, 128) * (unsigned)ngroups;
-  const int Lt = lat->dims[ND - 1];
-  if (herm)
-    wilson_full_kernel<ND, NC, true, R><<<grid, 128, 0, st>>>(lat->d_tab, (int)lat->V, Lt, kappa, bcr, bci,
-                                                             (const double2*)gauge, (const double2*)in,
-                                                             (double2*)out, ngroups);
-  else
-    wilson_full_kernel<ND, NC, false, R><<<grid, 128, 0, st>>>(lat->d_tab, (int)lat->V, Lt, kappa, bcr, bci,
-                                                              (const double2*)gauge, (const double2*)in,
-                                                              (double2*)out, ngroups);
+  if constexpr (ND == 4) {
+    const int64_t n = lat->V * ngroups, wave8 = 148 * 8 * 32, wave12 = 148 * 12 * 32;  // threads per wave
+    if (n > 2 * wave8 || (n > wave8 && n <= wave12))
+      return launch_form<ND, NC, R, 64, 6>(lat, kappa, herm, bcr, bci, gauge, ngroups, in, out, st);
+  }
+  launch_form<ND, NC, R, 128, 1>(lat, kappa, herm, bcr, bci, gauge, ngroups, in, out, st);
 }
 
-// nvec vectors: groups of R = 2 (4D, four-component spinors) or 4 (2D, 3D) vectors
-// per thread share each link load (sized to the 255-register budget), the groups of
-// a site block in consecutive blocks; a remainder runs one vector per thread.
-// Measured at 32^4 SU(3), 4 vectors: 0.43 of the HBM peak with R = 2, 0.39 with
-// R = 1 (one vector alone: 0.66-0.69) -- the kernel is latency-bound at 8 warps per SM.
+// nvec vectors: in two and three dimensions groups of four vectors per thread share each
+// link load, the groups of a site block in consecutive blocks; a remainder runs one vector
+// per thread.
 template <int ND, int NC>
 static int launch_full(const lym_lattice* lat, double kappa, int herm, double bcr, double bci,
                        const void* gauge, int nvec, const void* in, void* out, cudaStream_t st) {
-  constexpr int R = ND == 4 ? 2 : 4;
+  constexpr int R = ND == 4 ? 1 : 4;
   const size_t vec = (size_t)Gamma<ND>::NS * NC * lat->V * sizeof(double2);
   const int ng = nvec / R;
   if (ng > 0) launch_full_r<ND, NC, R>(lat, kappa, herm, bcr, bci, gauge, ng, in, out, st);
