@@ -305,6 +305,12 @@ int lym_momenta_kick(int64_t n, const void* momenta, const void* force, double e
 int lym_link_drift(int nd, int nc, int64_t volume, const void* gauge, const void* momenta, double eps,
                    int reunitarize, void* out, void* stream);
 
+/* A gauge kick and the drift after it in one pass: momenta_out = momenta + eps_p * F_gauge(gauge),
+ * gauge_out = expm(eps_u momenta_out) gauge.  gauge_out is another field than gauge (the force
+ * reads neighbouring links); momenta_out may be momenta. */
+int lym_gauge_kick_drift(const lym_lattice* lat, int nc, double beta, const void* gauge, const void* momenta,
+                         double eps_p, double eps_u, void* momenta_out, void* gauge_out, void* stream);
+
 /* The gauge part of an HMC step on nlat independent lattices (each its own lattice
  * object, N, beta, links gauges[l] and momenta momenta[l], reference layout) in two
  * launches whatever their sizes and (nd, N): momenta += eps_p * F_gauge(U) for every

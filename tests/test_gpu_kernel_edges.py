@@ -250,3 +250,33 @@ def test_lattices_of_uneven_sizes_together(cuda_device, geoms, nc, precision):
                                                            refs[k][2])) / np.linalg.norm(bs[k][i])
             assert res < tols[k], (k, i, reports[k][i])
             assert reports[k][i]["status"] == 0
+
+
+# the last two lie on either side of the size from which 4D SU(3) runs blocks of eight warps
+@pytest.mark.parametrize("geom,nc", [((7, 3), 3), ((3, 5, 2), 2), ((4, 3, 2, 33), 2), ((3, 1, 5, 7), 3),
+                                     ((7, 9, 28, 32), 3), ((7, 9, 30, 31), 3)])
+def test_kick_and_drift_in_one_pass(cuda_device, geom, nc):
+    """Momenta and links after one gauge kick and drift, the force alone and one smearing step.
+    Momenta and forces of order one per entry: exp(0.1 P) takes a few dozen more products; links
+    near the identity keep the projection well conditioned."""
+    from tfleonardym_b200 import gauge_action, smearing
+    from tfleonardym_b200 import lattice as lt
+    rng = np.random.default_rng(int(np.prod(geom)) + nc)
+    u, beta, eps_p, eps_u = smooth_links(rng, geom, nc, spread=0.05), 5.5, -0.15, 0.1
+    x = cnormal(rng, u.shape)
+    p = 0.5 * (x - np.conj(np.swapaxes(x, 1, 2)))
+    p -= np.einsum("miiv->mv", p)[:, None, None] * (np.eye(nc) / nc)[None, :, :, None]
+    tables = O.lookup_tables(geom)
+    force = O.gauge_force(u, beta, tables)
+    kicked = O.update_momenta(p, force, eps_p)
+    action = gauge_action.yang_mills(lt.Configuration(cu(u), geom, nc, len(geom)), beta)
+    given = cu(p)
+    p_out, u_out = action.kick_and_drift(given, eps_p, eps_u)
+    assert relerr(p_out.cpu().numpy(), kicked) < TOL
+    assert relerr(u_out.cpu().numpy(), O.update_link_field(u, kicked, eps_u)) < TOL
+    assert np.array_equal(given.cpu().numpy(), p)
+    assert np.array_equal(action.cfg.gauge_field.cpu().numpy(), u)
+    assert relerr(action.force().cpu().numpy(), force) < TOL
+    fat = smearing.ape_smearing(action.cfg, 0.3, len(geom) - 1)
+    fat = getattr(fat, "gauge_field", fat)
+    assert relerr(fat.cpu().numpy(), O.ape_smearing(u, tables, 0.3, len(geom) - 1)) < TOL

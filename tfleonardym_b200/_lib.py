@@ -85,6 +85,8 @@ SIGNATURES = {
     "lym_plaquette_sum": (c_int, [c_void_p, c_int, c_void_p, P(c_double), c_void_p]),
     "lym_momenta_energy": (c_int, [c_int, c_int, c_int64, c_void_p, P(c_double), c_void_p]),
     "lym_gauge_kick": (c_int, [c_void_p, c_int, c_double, c_void_p, c_void_p, c_double, c_void_p, c_void_p]),
+    "lym_gauge_kick_drift": (c_int, [c_void_p, c_int, c_double, c_void_p, c_void_p, c_double, c_double, c_void_p,
+                                     c_void_p, c_void_p]),
     "lym_momenta_kick": (c_int, [c_int64, c_void_p, c_void_p, c_double, c_void_p, c_void_p]),
     "lym_link_drift": (c_int, [c_int, c_int, c_int64, c_void_p, c_void_p, c_double, c_int, c_void_p, c_void_p]),
     "lym_update_momenta": (c_int, [c_int64, c_void_p, c_void_p, c_double, c_void_p]),

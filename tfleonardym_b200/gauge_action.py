@@ -47,6 +47,16 @@ class yang_mills:  # noqa: N801 - reference name
                                              _dev.ptr(p), float(eps), _dev.ptr(out), _dev.stream()), "lym_gauge_kick")
         return out
 
+    def kick_and_drift(self, momenta, eps_p, eps_u):
+        """(momenta + eps_p * force(), exp(eps_u * those momenta) links) as new tensors, in one kernel."""
+        u = _dev.as_c128(self.cfg.gauge_field)
+        p = _dev.as_c128(momenta)
+        p_out, u_out = torch.empty_like(p), torch.empty_like(u)
+        _lib.check(_lib.lib().lym_gauge_kick_drift(_lat(self.cfg).handle, u.shape[1], float(self.beta), _dev.ptr(u),
+                                                   _dev.ptr(p), float(eps_p), float(eps_u), _dev.ptr(p_out),
+                                                   _dev.ptr(u_out), _dev.stream()), "lym_gauge_kick_drift")
+        return p_out, u_out
+
     def energy(self):
         re, _ = plaquette_trace_sum(self.cfg)
         return -self.beta * re / self.cfg.gauge_field.shape[1]

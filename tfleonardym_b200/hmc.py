@@ -154,7 +154,7 @@ def gauge_step_lattices(configs, momenta, betas, eps_p, eps_u):
 # list asks for exactly the force evaluations the reference makes.  The runner
 # sets an action's gauge configuration only when the links changed since it last
 # saw them, and applies each kick through the action's fused force-into-momenta
-# kernel where it has one.
+# kernel where it has one; a gauge kick and the drift after it are one kernel.
 # ---------------------------------------------------------------------------
 DRIFT, KICK = 0, 1
 
@@ -232,16 +232,27 @@ def _kick(action, momenta, w):
 def run_schedule(config, momenta, actions, ops, level_offset=0):
     """Run a compiled schedule; kick level l uses actions[level_offset + l]."""
     version, seen = 0, {}
-    for op in ops:
+    k = 0
+    while k < len(ops):
+        op = ops[k]
+        k += 1
         if op.kind == DRIFT:
             config = update_configuration(config, momenta, op.weight)
             version += 1
             continue
         a = level_offset + op.level
+        action = actions[a]
         if seen.get(a) != version:
-            actions[a].set_gauge_configuration(config)
+            action.set_gauge_configuration(config)
             seen[a] = version
-        momenta = _kick(actions[a], momenta, op.weight)
+        if type(action) is gauge_action.yang_mills and k < len(ops) and ops[k].kind == DRIFT:
+            momenta, links = action.kick_and_drift(momenta, op.weight, ops[k].weight)
+            config = lt.Configuration(gauge_field=links, geometry=config.geometry, colors=config.colors,
+                                      number_of_dimensions=config.number_of_dimensions)
+            version += 1
+            k += 1
+            continue
+        momenta = _kick(action, momenta, op.weight)
     return config, momenta
 
 
