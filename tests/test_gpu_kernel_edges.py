@@ -280,3 +280,52 @@ def test_kick_and_drift_in_one_pass(cuda_device, geom, nc):
     fat = smearing.ape_smearing(action.cfg, 0.3, len(geom) - 1)
     fat = getattr(fat, "gauge_field", fat)
     assert relerr(fat.cpu().numpy(), O.ape_smearing(u, tables, 0.3, len(geom) - 1)) < TOL
+
+
+# sites per parity: less than one block, ragged blocks; 23 and 24 sources on 25 blocks lie on either
+# side of the line (592 blocks) to the form with three blocks per SM
+@pytest.mark.parametrize("geom,nc,nrhs", [((2, 2), 3, 2), ((10, 16), 2, 3), ((6, 6, 10), 3, 2), ((6, 22), 2, 1),
+                                          ((4, 4, 4, 6), 3, 3), ((2, 10, 6, 10), 2, 5), ((8, 8, 10, 10), 2, 23),
+                                          ((8, 8, 10, 10), 2, 24)])
+def test_fp64_solves_launch_by_launch(cuda_device, geom, nc, nrhs):
+    """True residuals by the oracle; a forced tile keeps the solve out of the one-launch form."""
+    from tfleonardym_b200 import dirac_solver
+    rng = np.random.default_rng(int(np.prod(geom)) + nc + nrhs)
+    nd, vol, kappa, tol = len(geom), int(np.prod(geom)), 0.11, 1e-10
+    u = smooth_links(rng, geom, nc)
+    ubc, tables = O.apply_time_bc(u, O.antiperiodic_field(geom, BC)), O.lookup_tables(geom)
+    b = cnormal(rng, (nrhs, 4 if nd == 4 else 2, nc, vol))
+    for herm in ([False] if nd == 3 else [False, True]):
+        op = make_op(u, geom, kappa, herm, "fundamental")
+        solver = dirac_solver.conjugate_gradient(tol=tol, precision="f64", delta=0.05, rhs_per_thread=1)
+        x = solver.solve(op, cu(b))
+        for i in range(nrhs):
+            res = np.linalg.norm(b[i] - O.wilson_apply(ubc, x[i].cpu().numpy(), kappa, herm, tables))
+            assert res < tol * np.linalg.norm(b[i]), (herm, i, solver.reports[i])
+            assert solver.reports[i]["status"] == 0
+
+
+@pytest.mark.parametrize("nc", [2, 3])
+@pytest.mark.parametrize("values", [(1, 1, 1), (1, 1, 0.3), (1, 0.3, 0.3), (1, 0.99999, 0.9), (1, 0.5, 0.2),
+                                    (1, 0.3, 0.23), (1, 0.5, 1e-2), (1, 1e-3, 1e-3), (1, 0.7, 1e-6)])
+def test_projection_over_singular_values(cuda_device, nc, values):
+    """Polar factors of matrices with given singular values (equal ones, the line between the
+    two SU(3) forms, nearly singular ones), scales from 1e-6 to 1e6 and determinants of every
+    phase. The factor is conditioned by the smallest singular value: about thirty roundings of
+    1.1e-16 each, three times that times the condition number."""
+    from tfleonardym_b200 import smearing
+    rng = np.random.default_rng(nc)
+    vol = 333
+    u, v = (np.linalg.qr(cnormal(rng, (vol, nc, nc)))[0] for _ in range(2))
+    s = np.array((values[0], values[2]) if nc == 2 else values)
+    w = u @ v
+    phase = np.exp(1j * (np.linspace(-0.99 * np.pi, 0.99 * np.pi, vol) - np.angle(np.linalg.det(w))) / nc)
+    u *= phase[:, None, None]
+    w *= phase[:, None, None]
+    x = (u * s) @ v * 10.0 ** np.linspace(-6, 6, vol)[:, None, None]
+    got = smearing.unitary_sqrt_projection(cu(np.transpose(x, (1, 2, 0))[None])).cpu().numpy()[0]
+    det = np.linalg.det(w)
+    want = np.transpose(w / np.exp(1j * np.angle(det) / nc)[:, None, None], (1, 2, 0))
+    assert np.abs(got - want).max() < 1e-14 * max(values) / min(values)
+    g = np.transpose(got, (2, 0, 1))
+    assert np.abs(np.conj(np.swapaxes(g, 1, 2)) @ g - np.eye(nc)).max() < 1e-14

@@ -390,6 +390,96 @@ LYM_D Mat<3> expm(const Mat<3>& X) {
 template <int NC>
 LYM_D double inv_root(double d2) { return NC == 2 ? rsqrt(sqrt(d2)) : rcbrt(sqrt(d2)); }
 
+// A Hermitian 3 x 3 matrix: its diagonal, and (0,1), (0,2), (1,2)
+struct Herm3 {
+  double d[3];
+  cx<double> a, b, c;
+};
+
+// U^dag U
+LYM_D Herm3 gram(const Mat<3>& U) {
+  Herm3 H{};
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) H.d[j] += norm2(U.m[k][j]);
+    cmac_cj(H.a, U.m[k][0], U.m[k][1]);
+    cmac_cj(H.b, U.m[k][0], U.m[k][2]);
+    cmac_cj(H.c, U.m[k][1], U.m[k][2]);
+  }
+  return H;
+}
+
+// U <- U (a0 + a1 K + a2 K^2); with ADD, U + that, rounding a small correction once
+template <bool ADD>
+LYM_D void times_quadratic(Mat<3>& U, const Herm3& K, double a0, double a1, double a2) {
+  const double na = norm2(K.a), nb = norm2(K.b), nc = norm2(K.c);
+  Herm3 P;
+  P.d[0] = fma(a2, fma(K.d[0], K.d[0], na + nb), fma(a1, K.d[0], a0));
+  P.d[1] = fma(a2, fma(K.d[1], K.d[1], na + nc), fma(a1, K.d[1], a0));
+  P.d[2] = fma(a2, fma(K.d[2], K.d[2], nb + nc), fma(a1, K.d[2], a0));
+  P.a = fma(a2, K.d[0] + K.d[1], a1) * K.a + a2 * cmul_cj(K.c, K.b);
+  P.b = fma(a2, K.d[0] + K.d[2], a1) * K.b + a2 * (K.a * K.c);
+  P.c = fma(a2, K.d[1] + K.d[2], a1) * K.c + a2 * cmul_cj(K.a, K.b);
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    const cx<double> x = U.m[i][0], y = U.m[i][1], z = U.m[i][2];
+    cx<double> t = P.d[0] * x, u = P.d[1] * y, v = P.d[2] * z;
+    cmac_cj(t, P.a, y);
+    cmac_cj(t, P.b, z);
+    cmac(u, x, P.a);
+    cmac_cj(u, P.c, z);
+    cmac(v, x, P.b);
+    cmac(v, y, P.c);
+    U.m[i][0] = ADD ? x + t : t;
+    U.m[i][1] = ADD ? y + u : u;
+    U.m[i][2] = ADD ? z + v : v;
+  }
+}
+
+// U <- U p(U^dag U) near the unitary polar factor, p the quadratic through x^(-1/2) at the three
+// eigenvalues of U^dag U.  Any p positive there keeps the polar factor, and the product is formed
+// in FP64, so the eigenvalues (the trigonometric solution of the characteristic cubic) and p's
+// coefficients (divided differences of x^(-1/2), closed forms in the square roots) need no more
+// than FP32: they set how close the step lands, about 1e-7.  False, U as it was, where the
+// smallest eigenvalue is under 0.05 of the mean (beyond, the quadratic's cancellations would show) or the matrix is not finite.
+LYM_D bool polar_step_exact(Mat<3>& U) {
+  Herm3 K = gram(U);
+  const double m = (K.d[0] + K.d[1] + K.d[2]) * (1.0 / 3.0), inv = 1.0 / m;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) K.d[j] = fma(K.d[j], inv, -1.0);
+  K.a = inv * K.a;
+  K.b = inv * K.b;
+  K.c = inv * K.c;
+  const float d0 = (float)K.d[0], d1 = (float)K.d[1], d2 = (float)K.d[2];
+  const cx<float> a{(float)K.a.re, (float)K.a.im}, b{(float)K.b.re, (float)K.b.im}, c{(float)K.c.re, (float)K.c.im};
+  const float na = norm2(a), nb = norm2(b), nc = norm2(c);
+  const float q = (d0 * d0 + d1 * d1 + d2 * d2 + 2.f * (na + nb + nc)) * (1.f / 6.f);
+  const cx<float> ac = a * c;
+  const float dt = d0 * d1 * d2 + 2.f * (ac.re * b.re + ac.im * b.im) - d0 * nc - d1 * nb - d2 * na;
+  const float h = sqrtf(q);
+  const float r = q > 1e-16f ? fminf(1.f, fmaxf(-1.f, dt / (2.f * q * h))) : 0.f;
+  const float phi = acosf(r) * (1.f / 3.f);
+  const float k1 = 2.f * h * cosf(phi), k3 = 2.f * h * cosf(phi + 2.0943951f), k2 = -k1 - k3;
+  if (!(1.f + k3 > 0.05f) || !(k1 < 3.f)) return false;
+  const float s1 = sqrtf(1.f + k1), s2 = sqrtf(1.f + k2), s3 = sqrtf(1.f + k3);
+  const float f12 = -1.f / (s1 * s2 * (s1 + s2));
+  const float f123 = (s1 + s2 + s3) / (s1 * s2 * s3 * (s1 + s2) * (s2 + s3) * (s1 + s3));
+  const double sc = rsqrt(m);
+  times_quadratic<false>(U, K, sc * (double)(1.f / s1 - f12 * k1 + f123 * k1 * k2),
+                         sc * (double)(f12 - f123 * (k1 + k2)), sc * (double)f123);
+  return true;
+}
+
+// One step of third order, U <- U (1 - E/2 + 3 E^2/8), E = U^dag U - 1; |E|^2
+LYM_D double polar_step_near(Mat<3>& U) {
+  Herm3 E = gram(U);
+#pragma unroll
+  for (int j = 0; j < 3; ++j) E.d[j] -= 1.0;
+  times_quadratic<true>(U, E, 0.0, -0.5, 0.375);
+  return E.d[0] * E.d[0] + E.d[1] * E.d[1] + E.d[2] * E.d[2] + 2.0 * (norm2(E.a) + norm2(E.b) + norm2(E.c));
+}
+
 // Unitary polar factor by the scaled Newton iteration
 // U <- (g U + U^{-dag} / g) / 2, g = |det U|^{-1/N} (Higham, "Functions of
 // Matrices", sec. 8.6), then division by the principal det^{1/N}
@@ -397,7 +487,7 @@ LYM_D double inv_root(double d2) { return NC == 2 ? rsqrt(sqrt(d2)) : rcbrt(sqrt
 // The iteration converges quadratically, |U_{k+1} - U| <= |U_k - U|^2 / 2 near the end, so
 // a step of squared length 1e-17 leaves an error of 1e-17 and is the last.
 template <int NC>
-LYM_D Mat<NC> polar_su(const Mat<NC>& X) {
+LYM_D Mat<NC> polar_newton(const Mat<NC>& X) {
   Mat<NC> Uk = X;
   cx<double> d = det(Uk);
   for (int it = 0; it < 40; ++it) {
@@ -423,6 +513,40 @@ LYM_D Mat<NC> polar_su(const Mat<NC>& X) {
   }
   const cx<double> r = principal_root(d, NC);
   return mscale(cdiv(cx<double>{1.0, 0.0}, r), Uk);
+}
+
+// out of line: few links take it, and inlined it costs the others registers
+__device__ __noinline__ Mat<3> polar_newton3(Mat<3> X) { return polar_newton<3>(X); }
+
+// d^(-1/3), principal root, for d on the unit circle to 1e-5: the angle in FP32, then Newton steps
+// on w^3 = d in FP64, w^(-2) from conj(w)^2 (each squares the distance: 1e-7, 1e-14, 1e-28)
+LYM_D cx<double> inv_cube_root_unit(cx<double> d) {
+  float sn, cs;
+  sincosf(atan2f((float)d.im, (float)d.re) * (1.f / 3.f), &sn, &cs);
+  cx<double> w{cs, sn};
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const cx<double> w2 = w * w;
+    const double f = (3.0 - 2.0 * norm2(w)) * (1.0 / 3.0);
+    w = (2.0 / 3.0) * w + f * cmul_cj(w2, d);
+  }
+  return conj(w);
+}
+
+// SU(3) starts from polar_step_exact and one third-order step, which leaves 5/16 |E|^3 <= 1e-17
+// where |E|^2 < 1e-11; the Newton steps then only serve ill-conditioned matrices.  The two cost
+// about 400 FP64 operations against 230 for each of five Newton steps: smearing step at
+// 24^3 x 48 459 us against 558 us, errors against 64-bit polar factors the same (rms 7e-16,
+// unitarity 2.8e-16).
+template <int NC>
+LYM_D Mat<NC> polar_su(const Mat<NC>& X) {
+  if constexpr (NC == 3) {
+    Mat<3> U = X;
+    if (polar_step_exact(U) && polar_step_near(U) < 1e-11) return mscale(inv_cube_root_unit(det(U)), U);
+    return polar_newton3(X);
+  } else {
+    return polar_newton<NC>(X);
+  }
 }
 
 template <int NC>
@@ -464,7 +588,7 @@ __global__ void __launch_bounds__(128) unitary_projection_kernel(int64_t nlinks,
 // One APE smearing step (smearing.py:34-51) per link: the staples without direction no_dir,
 // the fat link (rho / 6) S + (1 - rho) U (rho U + (1 - rho) U for no_dir) and its projection,
 // so the staples and the fat links never reach memory.  FP64-bound (the projection).
-// 24^3 x 48 SU(3): 565 us against 1108 us in separate passes (staples, four scaled
+// 24^3 x 48 SU(3): 459 us against 1108 us in separate passes (staples, four scaled
 // sums with their copies, projection).
 template <int ND, int NC, int BLOCK>
 __global__ void __launch_bounds__(BLOCK, BLOCK == 256 ? 2 : 4)
@@ -707,9 +831,9 @@ __global__ void __launch_bounds__(128) hmc_multi_kernel(const __grid_constant__ 
 // Link kernels whose 4D SU(3) form at 128 registers is worth blocks of eight warps: 64 sites
 // and their directions share an SM's L1, and the block's rows of loads go out together.  From
 // three waves of sixteen warps per SM on: force / kick and drift / smear in us with 256 | 128
-// threads, 16^3 x 32 85.3 / 127.8 / 148.5 | 90.1 / 138.1 / 178.8, 16^4 42.7 / 66.6 / 75.8 |
-// 45.1 / 70.3 / 87.1; below, 12^3 x 24 29.5 / 48.7 / 53.3 | 28.4 / 46.4 / 56.2, 8^4 8.1 / 11.8 /
-// 14.0 | 6.1 / 9.7 / 11.5.  SU(2) and fewer dimensions gain nothing (24^4 SU(2) 94.7 / 145.6 /
+// threads, 16^3 x 32 85.3 / 128.0 / 106.1 | 90.0 / 141.4 / 121.5, 16^4 42.7 / 66.9 / 53.1 |
+// 45.3 / 72.8 / 61.1; below, 12^3 x 24 29.5 / 48.1 / 37.5 | 28.5 / 45.8 / 41.0, 8^4 7.9 / 11.7 /
+// 10.3 | 5.9 / 9.6 / 9.1.  SU(2) and fewer dimensions gain nothing (24^4 SU(2) 94.7 / 145.6 /
 // 146 | 92.4 / 142.1 / 140).
 constexpr int64_t kWideFrom = 3 * 16 * 148;  // warps
 #define LYM_LINK_LAUNCH(KERNEL, lat, nc, st, ...)                                                                \
