@@ -16,14 +16,17 @@ def stream():
 
 
 def as_c128(t, name="tensor"):
-    """Return a contiguous complex128 CUDA tensor view/copy of ``t`` (DLPack producers accepted)."""
+    """Return a contiguous complex128 CUDA tensor view/copy of ``t`` (DLPack producers accepted).
+
+    Its memory holds its values: a lazy conjugate or sign, which torch keeps as a flag that
+    contiguous() passes on, is written out (into a copy; without a flag nothing is copied)."""
     if not isinstance(t, torch.Tensor):
         t = torch.from_dlpack(t)
     if not t.is_cuda:
         raise ValueError(f"{name} must be a CUDA tensor")
     if t.dtype != torch.complex128:
         t = t.to(torch.complex128)
-    return t.contiguous()
+    return t.contiguous().resolve_conj().resolve_neg()
 
 
 def ptr(t):

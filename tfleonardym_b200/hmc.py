@@ -139,6 +139,9 @@ def gauge_step_lattices(configs, momenta, betas, eps_p, eps_u):
     pp = (ctypes.c_void_p * n)(*[p.data_ptr() for p in ps])
     _lib.check(_lib.lib().lym_gauge_hmc_step_multi(n, lats, ncs, bs, up, pp, float(eps_p), float(eps_u),
                                                    _dev.stream()), "lym_gauge_hmc_step_multi")
+    for given, t in zip([c.gauge_field for c in configs] + list(momenta), us + ps):
+        if isinstance(given, torch.Tensor) and given.data_ptr() != t.data_ptr():
+            given.copy_(t)  # the kernels worked on a copy (another type, order or a lazy conjugate)
 
 
 # ---------------------------------------------------------------------------
