@@ -223,8 +223,18 @@ def force_evaluations(ops):
     return counts
 
 
+_gauge_force_into_momenta = gauge_action.yang_mills.force_into_momenta
+
+
+def _plain_gauge(action):
+    """Whether the action's kick is the gauge action's own: a subclass, or an object or class given
+    another force_into_momenta, keeps what it has."""
+    return (type(action) is gauge_action.yang_mills
+            and getattr(action.force_into_momenta, "__func__", None) is _gauge_force_into_momenta)
+
+
 def _kick(action, momenta, w):
-    if type(action) is gauge_action.yang_mills:  # a subclass may have its own force_into_momenta
+    if _plain_gauge(action):
         return action.kicked_momenta(momenta, w)
     fused = getattr(action, "force_into_momenta", None)
     if fused is not None:
@@ -248,7 +258,8 @@ def run_schedule(config, momenta, actions, ops, level_offset=0):
         if seen.get(a) != version:
             action.set_gauge_configuration(config)
             seen[a] = version
-        if type(action) is gauge_action.yang_mills and k < len(ops) and ops[k].kind == DRIFT:
+        # the drift is of config's links: an action that works on other ones drifts in its own pass
+        if k < len(ops) and ops[k].kind == DRIFT and _plain_gauge(action) and action.cfg is config:
             momenta, links = action.kick_and_drift(momenta, op.weight, ops[k].weight)
             config = lt.Configuration(gauge_field=links, geometry=config.geometry, colors=config.colors,
                                       number_of_dimensions=config.number_of_dimensions)
