@@ -26,7 +26,10 @@ def as_c128(t, name="tensor"):
         raise ValueError(f"{name} must be a CUDA tensor")
     if t.dtype != torch.complex128:
         t = t.to(torch.complex128)
-    return t.contiguous().resolve_conj().resolve_neg()
+    t = t.contiguous()
+    if t.is_conj() or t.is_neg():  # two flags to test cost half of what the two calls below do
+        t = t.resolve_conj().resolve_neg()
+    return t
 
 
 def ptr(t):
