@@ -193,8 +193,9 @@ typedef struct lym_solver_report {
  * and CG on M^dag M with FP64 reliable updates.  The reference's own solvers
  * (dirac_solver.py) reach the same x up to tolerance.  `reports` has nrhs
  * entries.  Small lattices run the whole solve in one launch, a cluster of blocks per rhs,
- * unless params force a tile (rhs_per_thread); the reports then say kernel_launches 1,
- * rhs_per_thread 1, compressed_links 0, mixed_fma 0.
+ * unless params force a tile (rhs_per_thread) or x overlaps the source of another rhs; the
+ * reports then say kernel_launches 1, rhs_per_thread 1, compressed_links 0, mixed_fma 0.
+ * x may be b or overlap it: every source is read before a solution is written over it.
  * Returns LYM_ERR_NOT_CONVERGED if any rhs missed tol. */
 int lym_wilson_solve(lym_gauge* g, double kappa, int nrhs, const void* b, void* x,
                      const lym_solver_params* params, lym_solver_report* reports, void* stream);
@@ -208,7 +209,7 @@ int lym_wilson_solve(lym_gauge* g, double kappa, int nrhs, const void* b, void* 
  * reliable updates and the odd-site reconstruction run per lattice.  One rhs per hop
  * thread (FP32: 12-real links when every lattice's links are SU(N); FP16: the
  * mixed-precision hop).  When every lattice is small, all rhs run in one launch as in
- * lym_wilson_solve.  `reports` has sum(nrhs) entries in lattice order.  No reference
+ * lym_wilson_solve, and as there sources and solutions may overlap.  `reports` has sum(nrhs) entries in lattice order.  No reference
  * counterpart (the reference solves one lattice per process). */
 int lym_wilson_solve_multi(int nlat, lym_gauge* const* gauges, const double* kappas, const double* tols,
                            const int* nrhs, const void* const* b, void* const* x,

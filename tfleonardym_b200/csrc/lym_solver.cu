@@ -1615,6 +1615,22 @@ static SmallLat small_lat(const Work& w, double kappa, const void* b, void* x, c
   return L;
 }
 
+// Whether a solution buffer covers sources of another right-hand side.  The resident solver reads
+// a right-hand side's source and writes its solution without waiting for the others, so such
+// calls go launch by launch, where every source is read first; x == b is each one's own.
+static bool crosses_sources(int nlat, const Work* const* w, const int* nrhs, const void* const* bs, void* const* xs) {
+  auto overlaps = [&](int l, int m) {
+    const size_t nb = sizeof(double2) * w[l]->g->ncomp * (size_t)w[l]->g->V * nrhs[l];
+    const size_t nx = sizeof(double2) * w[m]->g->ncomp * (size_t)w[m]->g->V * nrhs[m];
+    const uintptr_t b = (uintptr_t)bs[l], x = (uintptr_t)xs[m];
+    return b < x + nx && x < b + nb;
+  };
+  for (int l = 0; l < nlat; ++l)
+    for (int m = 0; m < nlat; ++m)
+      if (overlaps(l, m) && !(l == m && bs[l] == xs[l])) return true;
+  return false;
+}
+
 // Fills a call's reports from the device's; returns the status of the call.
 static int small_reports(const SmallReport* d, int n, int64_t launches, lym_solver_report* rep) {
   int status = LYM_OK;
@@ -1665,7 +1681,8 @@ static int cg_solve(lym_gauge* g, double kappa, int nrhs, const void* b, void* x
   // order the solve after the caller's prior work, and the caller's later work after the solve
   LYM_CUDA(cudaEventRecord(w.ev_in, caller));
   LYM_CUDA(cudaStreamWaitEvent(w.stream, w.ev_in, 0));
-  if (prm->rhs_per_thread == 0 && small_applies(g->nd, g->nc, sp, g->Vh, nrhs, 1, prm->max_iter))
+  if (prm->rhs_per_thread == 0 && small_applies(g->nd, g->nc, sp, g->Vh, nrhs, 1, prm->max_iter) &&
+      !crosses_sources(1, &wp, &nrhs, &b, &x))
     rc = cg_solve_small(w, kappa, nrhs, b, x, prm, rep, w.stream);
   else
     rc = cg_solve_on(w, g, kappa, nrhs, b, x, prm, rep, w.stream);
@@ -2139,7 +2156,10 @@ static int cg_solve_multi(int nlat, lym_gauge* const* gs, const double* kappas, 
     vh_max = std::max(vh_max, gs[l]->Vh);
     systems += nrhs[l];
   }
-  const bool small = prm->rhs_per_thread == 0 && small_applies(nd, nc, sp, vh_max, systems, nlat, prm->max_iter);
+  std::vector<const Work*> works;
+  for (const MultiLat& L : lats) works.push_back(L.w);
+  const bool small = prm->rhs_per_thread == 0 && small_applies(nd, nc, sp, vh_max, systems, nlat, prm->max_iter) &&
+                     !crosses_sources(nlat, works.data(), nrhs, bs, xs);
   for (int l = 0; l < nlat && !small; ++l) {
     Work& w = *lats[l].w;
     int pick = -1;
