@@ -192,9 +192,10 @@ typedef struct lym_solver_report {
  * (M = 1 - kappa^2 H_eo H_oe, builder-defined: the reference has no even-odd)
  * and CG on M^dag M with FP64 reliable updates.  The reference's own solvers
  * (dirac_solver.py) reach the same x up to tolerance.  `reports` has nrhs
- * entries.  Small lattices run the whole solve in one launch, a cluster of blocks per rhs,
- * unless params force a tile (rhs_per_thread) or x overlaps the source of another rhs; the
- * reports then say kernel_launches 1, rhs_per_thread 1, compressed_links 0, mixed_fma 0.
+ * entries.  Small lattices run the whole solve in one launch, a cluster of blocks per rhs
+ * (several launches where it takes thousands of iterations), unless params force a tile
+ * (rhs_per_thread) or x overlaps the source of another rhs; the reports then say
+ * kernel_launches 1 (or their number), rhs_per_thread 1, compressed_links 0, mixed_fma 0.
  * x may be b or overlap it: every source is read before a solution is written over it.
  * Returns LYM_ERR_NOT_CONVERGED if any rhs missed tol. */
 int lym_wilson_solve(lym_gauge* g, double kappa, int nrhs, const void* b, void* x,

@@ -14,6 +14,7 @@
 // cluster write them between barriers.
 #include <cooperative_groups.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "lym_small.cuh"
@@ -26,9 +27,11 @@ namespace cg = cooperative_groups;
 
 constexpr int kSmallThreads = 256;  // at most
 constexpr int kSmallMaxCtas = 8;  // portable cluster size
-// A launch ends by itself after max_iter iterations at the latest; a limit that would let
-// one run for seconds goes to the graph form, whose host loop can be interrupted.
-constexpr int kSmallMaxIter = 100000;
+// A launch cannot be interrupted, so it ends after this many iterations x sites per thread x
+// waves of clusters, and the host launches the rest: half a second at the 30 to 60 us that an
+// iteration with one site per thread takes at most.  A solve that converges takes some hundred
+// iterations, so the usual call stays one launch.
+constexpr int64_t kSmallStretch = 8192;
 
 // --- loads of fields that the cluster writes: plain, never the read-only path -----------
 template <int SP, int NCOMP>
@@ -171,7 +174,8 @@ LYM_D double cluster_sum(ClusterSum& cs, double v) {
 
 template <int ND, int NC, int SP>
 __global__ void __launch_bounds__(kSmallThreads, 1)
-    small_cg_kernel(const SmallLat* __restrict__ lats, int nlat, const __grid_constant__ SmallLat one) {
+    small_cg_kernel(const SmallLat* __restrict__ lats, int nlat, const __grid_constant__ SmallLat one, bool resume,
+                    int stop) {
   constexpr int NS = Gamma<ND>::NS, NCOMP = NS * NC;
   constexpr int GP = SP == SP64 ? SP64 : (SP == SP32 ? SP32 : SP16);
   constexpr int XP = (SP == SP16 || SP == SPB16) ? SP32 : SP;
@@ -198,55 +202,72 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
   const double k = L.kappa, k2 = k * k;
   const int64_t V = 2 * (int64_t)vh;
   ClusterSum cs{slots, warps, 0};
+  if (resume && !L.rep[rhs].going) return;  // all blocks of the cluster
   cluster_sync(single);  // every block of the cluster runs before its shared memory is written
 
-  // sources: even-odd form (gamma_d b for the hermitian system), |b|^2
-  double n = 0.0;
-  for (int i = tid; i < 2 * vh; i += T) {
-    const int par = i >= vh, cb = par ? i - vh : i;
-    int x[ND];
-    const int lex = eo_coords<ND>(L.g, cb, par, x);
-    cx<double> v[NCOMP];
-#pragma unroll
-    for (int c = 0; c < NCOMP; ++c) {
-      v[c] = ld(L.b + ((int64_t)rhs * NCOMP + c) * V + lex);
-      if (L.hermitian && c >= (NS / 2) * NC) v[c] = -v[c];
-      n += norm2(v[c]);
-    }
-    store_sp<SP64, NCOMP>(par ? L.bo : L.be, rhs, cb, v);
-  }
-  const double bnorm2 = cluster_sum(cs, n);
-  const double want = L.tol * L.tol * bnorm2;
-
-  // b' = b_e - kappa H_eo b_o; x = 0, so the first residual is q = b'
-  n = 0.0;
-  for (int i = tid; i < vh; i += T) {
-    cx<double> acc[NS][NC], v[NCOMP], z[NCOMP];
-    small_hop<ND, NC, SP64, SP64>(L.g, L.hg64, L.bo, rhs, i, 0, false, acc);
-    load_full<SP64, NCOMP>(L.be, rhs, i, v);
-    cx<RT> w[NCOMP];
-    cx<XR> xz[NCOMP];
-#pragma unroll
-    for (int c = 0; c < NCOMP; ++c) {
-      v[c] -= k * acc[c / NC][c % NC];
-      n += norm2(v[c]);
-      w[c] = {(RT)v[c].re, (RT)v[c].im};
-      z[c] = czero<double>();
-      xz[c] = czero<XR>();
-    }
-    store_sp<SP64, NCOMP>(L.bp, rhs, i, v);
-    store_sp<SP64, NCOMP>(L.x64, rhs, i, z);
-    if constexpr (SP != SP64) store_sp<XP, NCOMP>(L.xs, rhs, i, xz);
-    store_sp<SP, NCOMP>(L.t, rhs, i, w);
-  }
-  double q2 = cluster_sum(cs, n);
-
-  double prev_q2 = 0.0, rr = 0.0, alpha = 0.0, pause2 = 0.0, tres = 0.0;
+  double n, bnorm2, q2 = 0.0, prev_q2 = 0.0, rr = 0.0, alpha = 0.0, pause2 = 0.0, tres = 0.0;
   int iters = 0, updates = 0, pause_iter = 0;
   bool done = false, first = true, ran = false;  // ran: iterated since the last plan
+  bool going = false;
   // mode 2: r = M^dag t (t = the FP64 residual, rounded), then the plan of the next run of
   // iterations; 0: t = M p; 1: r -= alpha M^dag t, and the updates of x and p
   int mode = 2;
+  if (resume) {
+    const SmallReport& S = L.rep[rhs];
+    // the fields are where the last launch left them, ahead of t = M p
+    bnorm2 = S.bnorm2;
+    prev_q2 = S.prev_q2;
+    rr = S.rr;
+    pause2 = S.pause2;
+    tres = S.true_residual;
+    iters = S.iterations;
+    updates = S.updates;
+    pause_iter = S.pause_iter;
+    first = false;
+    ran = true;
+    mode = 0;
+  } else {
+    // sources: even-odd form (gamma_d b for the hermitian system), |b|^2
+    n = 0.0;
+    for (int i = tid; i < 2 * vh; i += T) {
+      const int par = i >= vh, cb = par ? i - vh : i;
+      int x[ND];
+      const int lex = eo_coords<ND>(L.g, cb, par, x);
+      cx<double> v[NCOMP];
+#pragma unroll
+      for (int c = 0; c < NCOMP; ++c) {
+        v[c] = ld(L.b + ((int64_t)rhs * NCOMP + c) * V + lex);
+        if (L.hermitian && c >= (NS / 2) * NC) v[c] = -v[c];
+        n += norm2(v[c]);
+      }
+      store_sp<SP64, NCOMP>(par ? L.bo : L.be, rhs, cb, v);
+    }
+    bnorm2 = cluster_sum(cs, n);
+
+    // b' = b_e - kappa H_eo b_o; x = 0, so the first residual is q = b'
+    n = 0.0;
+    for (int i = tid; i < vh; i += T) {
+      cx<double> acc[NS][NC], v[NCOMP], z[NCOMP];
+      small_hop<ND, NC, SP64, SP64>(L.g, L.hg64, L.bo, rhs, i, 0, false, acc);
+      load_full<SP64, NCOMP>(L.be, rhs, i, v);
+      cx<RT> w[NCOMP];
+      cx<XR> xz[NCOMP];
+#pragma unroll
+      for (int c = 0; c < NCOMP; ++c) {
+        v[c] -= k * acc[c / NC][c % NC];
+        n += norm2(v[c]);
+        w[c] = {(RT)v[c].re, (RT)v[c].im};
+        z[c] = czero<double>();
+        xz[c] = czero<XR>();
+      }
+      store_sp<SP64, NCOMP>(L.bp, rhs, i, v);
+      store_sp<SP64, NCOMP>(L.x64, rhs, i, z);
+      if constexpr (SP != SP64) store_sp<XP, NCOMP>(L.xs, rhs, i, xz);
+      store_sp<SP, NCOMP>(L.t, rhs, i, w);
+    }
+    q2 = cluster_sum(cs, n);
+  }
+  const double want = L.tol * L.tol * bnorm2;
   while (true) {
     const bool fwd = mode == 0;
     for (int i = tid; i < vh; i += T) {
@@ -313,6 +334,10 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
       }
       cluster_sync(single);
       if (!(rr < pause2 || iters >= L.max_iter || iters >= pause_iter)) {
+        if (iters >= stop) {
+          going = true;
+          break;
+        }
         mode = 0;
         continue;
       }
@@ -390,7 +415,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
   }
 
   // x_o = b_o - kappa H_oe x_e, both parities into the reference layout
-  for (int i = tid; i < vh; i += T) {
+  for (int i = tid; i < vh && !going; i += T) {
     cx<double> acc[NS][NC], v[NCOMP];
     int x[ND];
     load_full<SP64, NCOMP>(L.x64, rhs, i, v);
@@ -404,7 +429,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     for (int c = 0; c < NCOMP; ++c)
       st(L.x + ((int64_t)rhs * NCOMP + c) * V + lo, v[c] - k * acc[c / NC][c % NC]);
   }
-  if (tid == 0) L.rep[rhs] = SmallReport{tres, iters, updates, done ? 1 : 0, 0};
+  if (tid == 0)
+    L.rep[rhs] = SmallReport{tres, iters, updates, done ? 1 : 0, going ? 1 : 0, bnorm2, prev_q2, rr, pause2, pause_iter, 0};
   cluster_sync(single);  // no block leaves while its shared memory may still be read or written
 }
 
@@ -423,8 +449,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
 //   several lattices, whose graph form copies state per lattice at every wait: faster at
 //     every size measured, 84 systems on 21 4D SU(3) lattices up to 1536 sites per parity
 //     4447 / 6023 us in FP64 and 3653 / 9415 in FP32
-bool small_applies(int nd, int nc, int sp, int64_t vh, int systems, int lattices, int max_iter) {
-  if (max_iter > kSmallMaxIter) return false;
+bool small_applies(int nd, int nc, int sp, int64_t vh, int systems, int lattices) {
   if (lattices > 1 && vh <= 2048) return systems <= 1024;
   if (systems > 64) return false;
   if (sp == SP64) {
@@ -441,7 +466,8 @@ bool small_applies(int nd, int nc, int sp, int64_t vh, int systems, int lattices
 // 128, which double the systems in flight (16^3 SU(2) FP32, 8 rhs: 379 us a solve with
 // 256, 466 with 128; 16 rhs: 713 and 543).
 template <int ND, int NC, int SP>
-static int launch_small(int64_t vh, const SmallLat* lats, int nlat, const SmallLat& one, int systems, cudaStream_t st) {
+static int launch_small(int64_t vh, const SmallLat* lats, int nlat, const SmallLat& one, int systems, int round,
+                        cudaStream_t st) {
   int threads = 128, ctas = 1;
   if (vh <= kSmallThreads) {
     for (threads = 64; threads < vh;) threads *= 2;
@@ -468,19 +494,24 @@ static int launch_small(int64_t vh, const SmallLat* lats, int nlat, const SmallL
     }
     if (systems > n) cfg.blockDim = dim3(threads);
   }
-  LYM_CUDA(cudaLaunchKernelEx(&cfg, small_cg_kernel<ND, NC, SP>, lats, nlat, one));
+  // 256 threads of 255 registers per SM; clusters beyond those that fit run in further waves
+  const int64_t cluster = (int64_t)ctas * cfg.blockDim.x, fit = std::max<int64_t>(1, 148 * 256 / cluster);
+  const int64_t waves = (systems + fit - 1) / fit, sites = (vh + cluster - 1) / cluster;
+  const int64_t stop = (round + 1) * std::max<int64_t>(1, kSmallStretch / (waves * sites));
+  LYM_CUDA(cudaLaunchKernelEx(&cfg, small_cg_kernel<ND, NC, SP>, lats, nlat, one, round > 0,
+                              (int)std::min<int64_t>(stop, 0x7fffffff)));
   return LYM_OK;
 }
 
 int small_launch(int nd, int nc, int sp, int64_t vh, const SmallLat* lats, int nlat, const SmallLat& one, int systems,
-                 cudaStream_t st) {
+                 int round, cudaStream_t st) {
 #define LYM_SMALL(ND_, NC_)                                                                    \
   if (nd == ND_ && nc == NC_) {                                                                \
     switch (sp) {                                                                              \
-      case SP64: return launch_small<ND_, NC_, SP64>(vh, lats, nlat, one, systems, st);        \
-      case SP32: return launch_small<ND_, NC_, SP32>(vh, lats, nlat, one, systems, st);        \
-      case SP16: return launch_small<ND_, NC_, SP16>(vh, lats, nlat, one, systems, st);        \
-      default: return launch_small<ND_, NC_, SPB16>(vh, lats, nlat, one, systems, st);         \
+      case SP64: return launch_small<ND_, NC_, SP64>(vh, lats, nlat, one, systems, round, st); \
+      case SP32: return launch_small<ND_, NC_, SP32>(vh, lats, nlat, one, systems, round, st); \
+      case SP16: return launch_small<ND_, NC_, SP16>(vh, lats, nlat, one, systems, round, st); \
+      default: return launch_small<ND_, NC_, SPB16>(vh, lats, nlat, one, systems, round, st); \
     }                                                                                          \
   }
   LYM_SMALL(2, 2)

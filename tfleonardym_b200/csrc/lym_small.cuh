@@ -8,7 +8,10 @@ namespace lym {
 
 struct SmallReport {
   double true_residual;
-  int iterations, updates, done, pad;
+  int iterations, updates, done;
+  int going;                              // stopped by the limit of the launch: the rest is where it goes on
+  double bnorm2, prev_q2, rr, pause2;
+  int pause_iter, pad;
 };
 
 // One lattice of a call: geometry, links, the fields of its workspace, and the system.
@@ -27,11 +30,13 @@ struct SmallLat {
 
 // Whether this form is the faster one for `systems` right-hand sides in all on `lattices`
 // lattices of at most vh sites per parity.
-bool small_applies(int nd, int nc, int sp, int64_t vh, int systems, int lattices, int max_iter);
+bool small_applies(int nd, int nc, int sp, int64_t vh, int systems, int lattices);
 
 // Launches the solves of nlat lattices with `systems` right-hand sides in all; `lats` is a
-// device array, or null with one lattice passed by value.
+// device array, or null with one lattice passed by value.  A launch ends after a bounded
+// number of iterations; right-hand sides whose report then says `going` go on from there in
+// the launch of the next `round` (from 0), which leaves the others as they are.
 int small_launch(int nd, int nc, int sp, int64_t vh, const SmallLat* lats, int nlat, const SmallLat& one, int systems,
-                 cudaStream_t st);
+                 int round, cudaStream_t st);
 
 }  // namespace lym

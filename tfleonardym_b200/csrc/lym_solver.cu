@@ -1648,6 +1648,21 @@ static int small_reports(const SmallReport* d, int n, int64_t launches, lym_solv
   return status;
 }
 
+// The launches of a call (one, unless right-hand sides reach the limit of a launch), the device's
+// reports d through the pinned h, and rep; returns the status of the call.
+static int small_solve(int nd, int nc, int sp, int64_t vh, const SmallLat* lats, int nlat, const SmallLat& one,
+                       int systems, const SmallReport* d, SmallReport* h, lym_solver_report* rep, cudaStream_t st) {
+  for (int round = 0;; ++round) {
+    const int rc = small_launch(nd, nc, sp, vh, lats, nlat, one, systems, round, st);
+    if (rc) return rc;
+    LYM_CUDA(cudaMemcpyAsync(h, d, sizeof(SmallReport) * systems, cudaMemcpyDeviceToHost, st));
+    LYM_CUDA(cudaStreamSynchronize(st));
+    bool going = false;
+    for (int i = 0; i < systems; ++i) going = going || h[i].going;
+    if (!going) return small_reports(h, systems, round + 1, rep);
+  }
+}
+
 static int cg_solve_small(Work& w, double kappa, int nrhs, const void* b, void* x, const lym_solver_params* prm,
                           lym_solver_report* rep, cudaStream_t st) {
   w.kappa = kappa;
@@ -1655,11 +1670,8 @@ static int cg_solve_small(Work& w, double kappa, int nrhs, const void* b, void* 
   static_assert(sizeof(SmallReport) <= 8 * sizeof(double), "the workspace keeps eight result doubles per rhs");
   SmallReport* d = reinterpret_cast<SmallReport*>(w.res);
   const SmallLat one = small_lat(w, kappa, b, x, prm, prm->tol, 0, d);
-  const int rc = small_launch(w.g->nd, w.g->nc, w.sp, w.Vh, nullptr, 1, one, nrhs, st);
-  if (rc) return rc;
-  LYM_CUDA(cudaMemcpyAsync(w.res_host, d, sizeof(SmallReport) * nrhs, cudaMemcpyDeviceToHost, st));
-  LYM_CUDA(cudaStreamSynchronize(st));
-  return small_reports(reinterpret_cast<const SmallReport*>(w.res_host), nrhs, 1, rep);
+  return small_solve(w.g->nd, w.g->nc, w.sp, w.Vh, nullptr, 1, one, nrhs, d, reinterpret_cast<SmallReport*>(w.res_host),
+                     rep, st);
 }
 
 static int cg_solve(lym_gauge* g, double kappa, int nrhs, const void* b, void* x, const lym_solver_params* prm,
@@ -1681,7 +1693,7 @@ static int cg_solve(lym_gauge* g, double kappa, int nrhs, const void* b, void* x
   // order the solve after the caller's prior work, and the caller's later work after the solve
   LYM_CUDA(cudaEventRecord(w.ev_in, caller));
   LYM_CUDA(cudaStreamWaitEvent(w.stream, w.ev_in, 0));
-  if (prm->rhs_per_thread == 0 && small_applies(g->nd, g->nc, sp, g->Vh, nrhs, 1, prm->max_iter) &&
+  if (prm->rhs_per_thread == 0 && small_applies(g->nd, g->nc, sp, g->Vh, nrhs, 1) &&
       !crosses_sources(1, &wp, &nrhs, &b, &x))
     rc = cg_solve_small(w, kappa, nrhs, b, x, prm, rep, w.stream);
   else
@@ -2158,7 +2170,7 @@ static int cg_solve_multi(int nlat, lym_gauge* const* gs, const double* kappas, 
   }
   std::vector<const Work*> works;
   for (const MultiLat& L : lats) works.push_back(L.w);
-  const bool small = prm->rhs_per_thread == 0 && small_applies(nd, nc, sp, vh_max, systems, nlat, prm->max_iter) &&
+  const bool small = prm->rhs_per_thread == 0 && small_applies(nd, nc, sp, vh_max, systems, nlat) &&
                      !crosses_sources(nlat, works.data(), nrhs, bs, xs);
   for (int l = 0; l < nlat && !small; ++l) {
     Work& w = *lats[l].w;
@@ -2194,11 +2206,8 @@ static int cg_solve_multi(int nlat, lym_gauge* const* gs, const double* kappas, 
       desc[l] = small_lat(w, kappas[l], bs[l], xs[l], prm, tols ? tols[l] : prm->tol, s0, drep + s0);
     }
     LYM_CUDA(cudaMemcpyAsync(lead.multi, desc, sizeof(SmallLat) * nlat, cudaMemcpyHostToDevice, st));
-    rc = small_launch(nd, nc, sp, vh_max, reinterpret_cast<SmallLat*>(lead.multi), nlat, desc[0], systems, st);
-    if (rc) return rc;
-    LYM_CUDA(cudaMemcpyAsync(lead.multi_host + dbytes, drep, rbytes, cudaMemcpyDeviceToHost, st));
-    LYM_CUDA(cudaStreamSynchronize(st));
-    return small_reports(reinterpret_cast<const SmallReport*>(lead.multi_host + dbytes), systems, 1, rep);
+    return small_solve(nd, nc, sp, vh_max, reinterpret_cast<SmallLat*>(lead.multi), nlat, desc[0], systems, drep,
+                       reinterpret_cast<SmallReport*>(lead.multi_host + dbytes), rep, st);
   }
   const double delta = prm->delta > 0 && prm->delta < 1 ? prm->delta : 0.1;
   const int chunk = prm->chunk > 0 ? std::min(prm->chunk, 256) : 8;
