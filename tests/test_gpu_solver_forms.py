@@ -162,3 +162,27 @@ def test_solves_that_converge_over_several_launches(cuda_device, precision):
     assert [r.true_residual for r in reps40] == [r.true_residual for r in reps[:40]]
     for s, b, x in zip(systems, bs, xs):
         assert max(s.residual(x[i], b[i]) for i in (0, 200, 511)) < 1.01 * tol
+
+
+@pytest.mark.parametrize("tiled", [0, 1])
+@pytest.mark.parametrize("precision", ["f64", "f32", "f16"])
+def test_solves_that_cannot_go_on_end(cuda_device, precision, tiled):
+    """A source that is not finite takes no step; the other right-hand sides converge and the call
+    returns, in both forms and on several lattices.  So does one whose residual falls to zero short
+    of its target."""
+    from tfleonardym_b200 import _lib
+    rng = np.random.default_rng(3)
+    systems = [System(rng, g, 2) for g in ((8, 12), (6, 10))]
+    bs = [s.sources(rng, 3) for s in systems]
+    bs[0][2, 0, 0, 5] = np.nan
+    bs[1][0, 1, 1, 7] = np.nan
+    want = [0, 0, _lib.LYM_ERR_NOT_CONVERGED, _lib.LYM_ERR_NOT_CONVERGED, 0, 0]
+    for n in (1, 2):
+        xs = [torch.empty_like(cu(b)) for b in bs[:n]]
+        rc, reps = solve_on(systems[:n], [cu(b) for b in bs[:n]], xs, precision, rhs_per_thread=tiled)
+        assert rc == _lib.LYM_ERR_NOT_CONVERGED and [r.status for r in reps] == want[:3 * n]
+        for s, b, x, st in zip(systems, bs, xs, (want[:3], want[3:])):
+            assert max(s.residual(x[i], b[i]) for i in range(3) if st[i] == 0) < TOL
+    x = torch.empty_like(cu(bs[0][:1]))
+    rc, reps = solve_on(systems[:1], [cu(bs[0][:1])], [x], precision, tol=1e-30, max_iter=2000, rhs_per_thread=tiled)
+    assert rc == _lib.LYM_ERR_NOT_CONVERGED and reps[0].iterations <= 2000

@@ -1736,6 +1736,7 @@ static int cg_solve_on(Work& w, lym_gauge* g, double kappa, int nrhs, const void
   std::vector<int> done(nrhs, 0), updates(nrhs, 0), restart(nrhs, 0);
   std::vector<double> target(nrhs, 0.0), tres(nrhs, 0.0), prev_q2(nrhs, 0.0), rate(nrhs, 0.0);
   std::vector<CGState> known(nrhs);
+  std::vector<int> planned(nrhs, -1);  // iterations at the last plan
   // sloppy runs get a reliable update at least this often, whatever the residual does
   const int max_interval = sp == SP64 ? (1 << 30) : 50;
   auto plan_rhs = [&](int i, double q2, double r2) -> void {
@@ -1758,7 +1759,9 @@ static int cg_solve_on(Work& w, lym_gauge* g, double kappa, int nrhs, const void
     S.rr = r2;
     S.pause2 = sp == SP64 ? est : std::max(est, delta * delta * r2);
     S.pause_iter = S.iters + max_interval;
-    S.active = S.iters >= S.max_iter ? 0 : 1;
+    // no step since the last plan (p = 0, or not finite): the next run would not take one either
+    S.active = S.iters >= S.max_iter || S.iters == planned[i] ? 0 : 1;
+    planned[i] = S.iters;
   };
   for (int i = 0; i < nrhs; ++i) {
     CGState& S = w.st_host[i];
@@ -2107,7 +2110,7 @@ struct MultiLat {
   int nreal = 0;
   double tol = 0;  // target true relative residual of this lattice
   std::vector<double> bnorm2, tres, prev_q2;
-  std::vector<int> done, updates, restart;
+  std::vector<int> done, updates, restart, planned;
 };
 
 static void multi_plan(MultiLat& L, const lym_solver_params* prm, double delta, int i, double q2, double r2) {
@@ -2127,7 +2130,8 @@ static void multi_plan(MultiLat& L, const lym_solver_params* prm, double delta, 
   S.rr = r2;
   S.pause2 = sp == SP64 ? est : std::max(est, delta * delta * r2);
   S.pause_iter = S.iters + (sp == SP64 ? (1 << 30) : 50);
-  S.active = S.iters >= S.max_iter ? 0 : 1;
+  S.active = S.iters >= S.max_iter || S.iters == L.planned[i] ? 0 : 1;
+  L.planned[i] = S.iters;
 }
 
 static int cg_solve_multi(int nlat, lym_gauge* const* gs, const double* kappas, const double* tols,
@@ -2310,6 +2314,7 @@ static int cg_solve_multi(int nlat, lym_gauge* const* gs, const double* kappas, 
     L.done.assign(n, 0);
     L.updates.assign(n, 0);
     L.restart.assign(n, 0);
+    L.planned.assign(n, -1);
     for (int i = 0; i < n; ++i) {
       std::memset(&w.st_host[i], 0, sizeof(CGState));
       w.st_host[i].max_iter = prm->max_iter;
