@@ -186,3 +186,15 @@ def test_solves_that_cannot_go_on_end(cuda_device, precision, tiled):
     x = torch.empty_like(cu(bs[0][:1]))
     rc, reps = solve_on(systems[:1], [cu(bs[0][:1])], [x], precision, tol=1e-30, max_iter=2000, rhs_per_thread=tiled)
     assert rc == _lib.LYM_ERR_NOT_CONVERGED and reps[0].iterations <= 2000
+
+
+# blocks: 81 each; three waves of two per SM instead of two of three in 4D SU(3) up to 888 (and from 1185),
+# the usual form between; SU(2) from 593 on
+@pytest.mark.parametrize("nc,nrhs", [(3, 7), (3, 8), (3, 11), (3, 12), (3, 16), (2, 12)])
+def test_fp64_solves_of_both_occupancies(cuda_device, nc, nrhs):
+    s = LargeSystem((12, 12, 12, 12), nc)
+    b = s.normal((nrhs,) + s.shape)
+    x = torch.empty_like(b)
+    rc, reps = solve_on([s], [b], [x], "f64")
+    assert rc == 0 and not one_launch(reps)
+    assert max(s.residual(x[i], b[i]) for i in range(nrhs)) < TOL

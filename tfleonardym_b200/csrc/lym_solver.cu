@@ -297,12 +297,16 @@ LYM_D void rhs_tile(const EoGeom& g, int& bx, int& by) {
 // 299 us, the solve 115 against 137 ms; FP16 (106 MB), 8 rhs, the solve 93.6 against
 // 98.5 ms.  16^4 (FP64 38 MB, 12 rhs): 66 us against 57 us the other way, FP16 16 rhs 20.2
 // against 17.6 us, so the slow tile stays below.
-constexpr unsigned kDenseFrom = 2 * 2 * 148;  // blocks: two waves of two per SM
-
 struct HopGrid {
   EoGeom g;
   dim3 grid;
-  bool dense() const { return grid.x * grid.y > kDenseFrom; }  // FP64 hop kernels: three blocks per SM
+  // FP64 hop kernels in the form with three blocks per SM: beyond two waves of two, and for
+  // 4D SU(3) below nine waves only where it saves a third of them or more.
+  bool dense(int nc) const {
+    const unsigned n = grid.x * grid.y, w2 = (n + 295) / 296, w3 = (n + 443) / 444;
+    if (g.nd == 4 && nc == 3 && w2 < 9) return w2 > 2 && 2 * w2 >= 3 * w3;
+    return w2 > 2;
+  }
   HopGrid(const EoGeom& geom, int nblk, int tiles, size_t link_bytes) : g(geom), grid(nblk, tiles) {
     if (tiles > 1 && nblk <= 65535 && link_bytes > (size_t)64 << 20) {
       g.tile_fast = 1;
@@ -389,12 +393,15 @@ __global__ void __launch_bounds__(128) norm64_kernel(int64_t Vh, EoField f, doub
 // Launch bounds of the hop kernels: FP64 ones declare one resident block per
 // SM as enough, which lets ptxas keep every neighbour's loads in flight at once
 // (about 250 registers, two blocks); the memory-bound FP64 hop runs ~20% faster at
-// 32^4 than with ptxas's default register target.  Beyond two full waves of blocks
-// (kDenseFrom) a form with three blocks per SM (168 registers, a few spilled) is the
-// faster one: 24^3 x 48, the FP64 solve 109 against 115 ms with 4 rhs and 36.5 against
-// 37.3 ms with one, the FP16 one (its FP64 updates) 90.2 against 93.4 ms with 8; at 16^4
-// with one rhs (256 blocks) it is 1.5 % slower.  Sloppy kernels keep ptxas's default
-// register target.
+// 32^4 than with ptxas's default register target.  Beyond two full waves of blocks a form
+// with three blocks per SM (168 registers, a few spilled) is the faster one (HopGrid::dense):
+// 24^3 x 48 SU(3), the FP64 solve 109 against 115 ms with 4 rhs and 36.5 against 37.3 ms with
+// one, the FP16 one (its FP64 updates) 90.2 against 93.4 ms with 8; at 16^4 with one rhs (256
+// blocks) it is 1.5 % slower.  FP64 solves, usual / dense, by blocks: SU(2) 12^4 648 1.02, 810
+// 1.06, 1296 1.07, 16^4 768 1.06, 2048 1.08; 2D 256^2 768 SU(2) 1.02, SU(3) 1.07, 1536 1.04,
+// 1.11; 3D 32^3 640 1.06, 1.04, 1280 1.14, 1.11.  4D SU(3), waves of two | of three: 3 | 2
+// 1.02 to 1.05, 4 | 3 0.98 to 1.03, 5 | 3 1.01 to 1.06, 6 | 4 1.01, 7 | 5 0.99.  Sloppy kernels keep
+// ptxas's default register target.
 //
 // The kernel bodies below take the block's site block `bx` and rhs tile `by`
 // (and, for the reductions, the site-block count nblk) so that the
@@ -956,7 +963,7 @@ struct Impl {
     const dim3 grid(w.nblk, w.nrhs);
     const HopGrid h = hop_tiles(w);
     const CGState* cst = w.st;
-    if (h.dense()) iterate_hops<DB>(w, st, h, cst, k2);
+    if (h.dense(NC)) iterate_hops<DB>(w, st, h, cst, k2);
     else iterate_hops<MB>(w, st, h, cst, k2);
     launch(w, st, cg_p_kernel<SP, XP, NCOMP>, grid, dim3(128), w.Vh, w.r, w.p, w.xs, w.st, w.counters);
   }
@@ -982,7 +989,7 @@ struct Impl {
       kernel<<<h.grid, 128, 0, st>>>(h.g, w.hg64, in, par, out, z0, z1, a1, c, w.upd, w.partials, w.counters, res,
                                      w.nblk);
     };
-#define LYM_H64(A, B) run(h.dense() ? hop64_lincomb_kernel<ND, NC, A, B, 3> : hop64_lincomb_kernel<ND, NC, A, B, 1>)
+#define LYM_H64(A, B) run(h.dense(NC) ? hop64_lincomb_kernel<ND, NC, A, B, 3> : hop64_lincomb_kernel<ND, NC, A, B, 1>)
     if (g5in && g5out) LYM_H64(true, true);
     else if (g5in) LYM_H64(true, false);
     else if (g5out) LYM_H64(false, true);
@@ -1026,7 +1033,7 @@ struct Impl {
   static void dslash(Work& w, cudaStream_t st) {
     const HopGrid h = hop_tiles(w);
     w.launches += 1;
-    auto hop = h.dense() ? cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX, DB>
+    auto hop = h.dense(NC) ? cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX, DB>
                          : cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX, MB>;
     hop<<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.p, w.s, 1, nullptr);
   }
@@ -1034,9 +1041,9 @@ struct Impl {
     const double k2 = w.kappa * w.kappa;
     const HopGrid h = hop_tiles(w);
     w.launches += 2;
-    auto hop = h.dense() ? cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX, DB>
+    auto hop = h.dense(NC) ? cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX, DB>
                          : cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX, MB>;
-    auto rnew = h.dense() ? cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX, DB> : cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX, MB>;
+    auto rnew = h.dense(NC) ? cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX, DB> : cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX, MB>;
     hop<<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.t, w.s, 1, nullptr);
     rnew<<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.s, w.t, w.r, k2, w.upd,
                                                                       w.partials, w.counters, w.res, w.nblk);
