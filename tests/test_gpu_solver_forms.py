@@ -198,3 +198,21 @@ def test_fp64_solves_of_both_occupancies(cuda_device, nc, nrhs):
     rc, reps = solve_on([s], [b], [x], "f64")
     assert rc == 0 and not one_launch(reps)
     assert max(s.residual(x[i], b[i]) for i in range(nrhs)) < TOL
+
+
+def test_hop_alone_after_a_one_launch_solve(cuda_device):
+    """lym_dslash_eo on a workspace that only one-launch solves have used: picks a hop form as a
+    launch-by-launch solve does, and the workspace solves on in both forms."""
+    from tfleonardym_b200 import _dev, _lib
+    rng = np.random.default_rng(14)
+    s = System(rng, (4, 4, 4, 8), 3)
+    b = s.sources(rng, 4)
+    for precision in ("f64", "f32", "f16"):
+        x = torch.empty_like(cu(b))
+        for tiled in (0, 1, 0):
+            rc, reps = solve_on([s], [cu(b)], [x], precision, rhs_per_thread=tiled)
+            assert rc == 0 and one_launch(reps) == (not tiled)
+            assert max(s.residual(x[i], b[i]) for i in range(4)) < TOL
+            handle = s.op.solver_gauge(() if precision == "f64" else (precision,))
+            assert _lib.lib().lym_dslash_eo(handle, _lib.PREC[precision], 4, 3, _dev.stream()) == 0
+        assert _lib.lib().lym_dslash_eo(handle, _lib.PREC[precision], 999, 1, _dev.stream()) == _lib.LYM_ERR_BAD_ARG

@@ -461,7 +461,7 @@ bool small_applies(int nd, int nc, int sp, int64_t vh, int systems, int lattices
 }
 
 // Threads per block and blocks per cluster.  Up to 256 sites one block, whose barriers cost
-// almost nothing; then one site per thread in blocks of 128 (two per SM by registers);
+// almost nothing; then one site per thread in four or eight blocks of 128 (two per SM by registers);
 // above 1024 sites eight blocks of 256 while all clusters are resident at once, else of
 // 128, which double the systems in flight (16^3 SU(2) FP32, 8 rhs: 379 us a solve with
 // 256, 466 with 128; 16 rhs: 713 and 543).
@@ -472,7 +472,7 @@ static int launch_small(int64_t vh, const SmallLat* lats, int nlat, const SmallL
   if (vh <= kSmallThreads) {
     for (threads = 64; threads < vh;) threads *= 2;
   } else {
-    while (ctas < kSmallMaxCtas && (int64_t)ctas * threads < vh) ctas *= 2;
+    for (ctas = 4; ctas < kSmallMaxCtas && (int64_t)ctas * threads < vh;) ctas *= 2;  // two hold 256 sites
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(systems * ctas));

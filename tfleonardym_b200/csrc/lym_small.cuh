@@ -23,7 +23,7 @@ struct SmallLat {
   const double2* b;                       // sources and solutions, reference layout (nrhs, ns, N, V)
   double2* x;
   double kappa, tol, delta;
-  int hermitian, max_iter, nrhs;
+  int hermitian, max_iter;
   int sys0;                               // first right-hand side of this lattice in the launch
   SmallReport* rep;                       // of the lattice's right-hand sides
 };

@@ -881,6 +881,7 @@ struct Work {
   int R = 1;                     // right-hand sides per thread in the hop kernels (autotuned)
   int mx = 0;                    // FP16 hop arithmetic: 0 FP32 (hop_tile), 1 mixed (hop_tile_mx)
   bool tuned = false;
+  bool picked = false;            // a solve or the autotuner has selected a hop form
   int tuned_i = 0;
   // hop-kernel candidates: right-hand sides per thread x compressed / full links
   // (x FP32 / mixed-precision arithmetic for FP16)
@@ -1474,6 +1475,7 @@ static int build_graph(Work& w, int chunk, cudaStream_t st) {
 // precision hop when forced_mx and the precision is FP16.
 static void select_cand(Work& w, int i) {
   w.cur = i;
+  w.picked = true;
   w.ops = w.ops_r[i];
   w.R = w.rcand[i];
   w.mx = w.mcand[i];
@@ -1616,7 +1618,6 @@ static SmallLat small_lat(const Work& w, double kappa, const void* b, void* x, c
   L.delta = prm->delta > 0 && prm->delta < 1 ? prm->delta : 0.1;
   L.hermitian = prm->hermitian ? 1 : 0;
   L.max_iter = prm->max_iter;
-  L.nrhs = w.nreal;
   L.sys0 = sys0;
   L.rep = rep;
   return L;
@@ -2453,6 +2454,12 @@ static int dslash_eo(lym_gauge* g, int precision, int nrhs, int repeats, cudaStr
   Work* w = find_work(g, nrhs, precision);
   LYM_REQUIRE(w, LYM_ERR_BAD_ARG,
               "no solver workspace for precision %d and %d right-hand sides", precision, nrhs);
+  if (!w->picked) {
+    // only one-launch solves so far, which choose no hop form: take the one that the iterations
+    // of a launch-by-launch solve would
+    const int rc = autotune(*w, st, 0, 0, 0);
+    if (rc) return rc;
+  }
   for (int i = 0; i < repeats; ++i) w->ops.dslash(*w, st);
   LYM_CHECK_LAUNCH();
   return LYM_OK;
