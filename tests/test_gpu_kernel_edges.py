@@ -329,3 +329,23 @@ def test_projection_over_singular_values(cuda_device, nc, values):
     assert np.abs(got - want).max() < 1e-14 * max(values) / min(values)
     g = np.transpose(got, (2, 0, 1))
     assert np.abs(np.conj(np.swapaxes(g, 1, 2)) @ g - np.eye(nc)).max() < 1e-14
+
+
+# threads of single vectors: 64152 and 72171 (between the waves of 56832 and 75776 threads), 131072
+# (between the second and the third of them), 207360 (SU(2) takes pairs up to the third wave); an odd count
+# stays with single vectors
+@pytest.mark.parametrize("geom,nc,nvec", [((9, 9, 9, 11), 3, 8), ((9, 9, 9, 11), 2, 8), ((9, 9, 9, 11), 3, 9),
+                                          ((8, 8, 8, 16), 3, 16), ((12, 12, 12, 12), 2, 10), ((12, 12, 12, 12), 3, 10)])
+def test_operator_on_pairs_of_vectors(cuda_device, geom, nc, nvec):
+    rng = np.random.default_rng(nvec + nc)
+    vol = int(np.prod(geom))
+    u = links(rng, geom, nc, unitary=False)
+    ubc, tables = O.apply_time_bc(u, O.antiperiodic_field(geom, BC)), O.lookup_tables(geom)
+    x = cnormal(rng, (nvec, 4, nc, vol))
+    for herm in (False, True):
+        op = make_op(u, geom, 0.12, herm, "fundamental")
+        out = op.apply(cu(x)).cpu().numpy()
+        for k in (0, nvec // 2, nvec - 1):
+            assert relerr(out[k], O.wilson_apply(ubc, x[k], 0.12, herm, tables)) < TOL, (herm, k)
+        for k in range(nvec):
+            assert relerr(out[k], op.apply(cu(x[k])).cpu().numpy()) < TOL, (herm, k)

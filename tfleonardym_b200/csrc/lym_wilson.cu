@@ -207,12 +207,27 @@ static void launch_full_r(const lym_lattice* lat, double kappa, int herm, double
 
 // nvec vectors: in two and three dimensions groups of four vectors per thread share each
 // link load, the groups of a site block in consecutive blocks; a remainder runs one vector
-// per thread.
+// per thread.  In four dimensions one vector per thread, but two (half the threads, 8 warps
+// of 254 registers per SM) for an even nvec whose pairs run fewer waves than single vectors
+// at 12 warps do, up to two waves of them for SU(3) and three for SU(2), beyond which the
+// occupancy wins.  us for pairs | single vectors: SU(3) 8^3 x 16 8 vectors 14.6 | 16.7,
+// 12^4 6 23.5 | 26.9, 16^3 x 8 4 25.0 | 26.9 (outside: 10 vectors 64.5 | 57.3, 16^4 4
+// 55.6 | 49.5); SU(2) 16^3 x 8 2 8.5 | 10.5, 12^4 6 14.7 | 16.4, 10 20.8 | 22.8 (outside:
+// 16^4 6 43.4 | 41.2, 12^4 8 20.3 | 18.7).
 template <int ND, int NC>
 static int launch_full(const lym_lattice* lat, double kappa, int herm, double bcr, double bci,
                        const void* gauge, int nvec, const void* in, void* out, cudaStream_t st) {
   constexpr int R = ND == 4 ? 1 : 4;
   const size_t vec = (size_t)Gamma<ND>::NS * NC * lat->V * sizeof(double2);
+  if constexpr (ND == 4) {
+    const int64_t n = lat->V * nvec, wave = 148 * 8 * 32 * 2, wave1 = 148 * 12 * 32;  // vectors' sites per wave
+    const int64_t waves = (n + wave - 1) / wave;
+    if (nvec % 2 == 0 && waves < (n + wave1 - 1) / wave1 && waves <= (NC == 3 ? 2 : 3)) {
+      launch_form<ND, NC, 2, 128, 1>(lat, kappa, herm, bcr, bci, gauge, nvec / 2, in, out, st);
+      LYM_CHECK_LAUNCH();
+      return LYM_OK;
+    }
+  }
   const int ng = nvec / R;
   if (ng > 0) launch_full_r<ND, NC, R>(lat, kappa, herm, bcr, bci, gauge, ng, in, out, st);
   const int rest = nvec - ng * R;
