@@ -216,3 +216,18 @@ def test_hop_alone_after_a_one_launch_solve(cuda_device):
             handle = s.op.solver_gauge(() if precision == "f64" else (precision,))
             assert _lib.lib().lym_dslash_eo(handle, _lib.PREC[precision], 4, 3, _dev.stream()) == 0
         assert _lib.lib().lym_dslash_eo(handle, _lib.PREC[precision], 999, 1, _dev.stream()) == _lib.LYM_ERR_BAD_ARG
+
+
+# blocks of the operator kernels: 324 and 392 (one wave of three per SM instead of two of two) and 640 (two
+# instead of three); the usual form for 314 in 2D SU(2), 768 in 4D SU(3) and 512
+@pytest.mark.parametrize("geom,nc", [((12, 12, 12, 24), 3), ((12, 12, 12, 24), 2), ((224, 224), 2), ((200, 200), 2),
+                                     ((16, 16, 16, 20), 3), ((16, 16, 16, 24), 3), ((16, 16, 16, 16), 3)])
+def test_multishift_of_both_occupancies(cuda_device, geom, nc):
+    from tfleonardym_b200 import dirac, dirac_solver
+    s = LargeSystem(geom, nc, hermitian=True)
+    b = s.normal(s.shape)
+    shifts = [0.05, 0.4, 2.0]
+    xs = dirac_solver.multishift_cg(5000, TOL, precision="f64").solve(dirac.SquareOperator(s.op), b, shifts)
+    for x, shift in zip(xs, shifts):
+        res = b - s.op.apply(s.op.apply(x)) - shift * x
+        assert float(torch.linalg.vector_norm(res) / torch.linalg.vector_norm(b)) < TOL * 1.01

@@ -748,13 +748,19 @@ struct MsImpl {
     dim3 tile(2 * w.nblk, w.G / R), grid(2 * w.nblk, w.G);
     // FP64 kernels hold about 250 registers, two blocks per SM; where that leaves a last wave
     // nearly empty, the form with three blocks per SM (168 registers, a few spilled) runs
-    // fewer waves of about 1.2 times the length.  12^3 x 24, one source (324 blocks, two
-    // waves or one): 12.8 and 15.4 us against 16.6 and 19.0 us, the solve 8.5 against 9.8 ms;
-    // at one wave of each (8^3 x 16) or several (16^4, 24^3 x 48) it is 2 to 13 % slower.
+    // fewer waves of about 1.2 times the length.  One wave instead of two (297 to 444 blocks;
+    // 4D SU(3) 12^3 x 24, 324 blocks: 12.8 and 15.4 us a kernel against 16.6 and 19.0 us):
+    // force 6.75 | 7.77 ms, 14^3 x 20 7.58 | 8.61, SU(2) 12^3 x 24 6.04 | 6.73, 2D SU(3) 200^2
+    // 1.49 | 1.57; in 2D SU(2) 200^2 (314 blocks) 1.348 | 1.312, 224^2 (392) 1.367 | 1.403.
+    // Two instead of three (593 to 888): 4D SU(3) 640 blocks 12.80 | 13.14, but 768 14.97 | 14.85
+    // and 832 16.61 | 16.34; SU(2) 768 10.49 | 11.13, 2D SU(3) 648 to 800 blocks 5 % faster,
+    // SU(2) 1 to 3 %.  Otherwise (8^3 x 16, 16^4, 16^3 x 18, 24^3 x 48) it is 2 to 13 % slower.
     bool dense = false;
     if constexpr (SP == SP64) {
       const int n = 2 * w.nblk * (w.G / R), w2 = (n + 295) / 296, w3 = (n + 443) / 444;
-      dense = w2 <= 3 && 5 * w2 > 6 * w3;
+      dense = w2 <= 3 && w3 < w2;
+      if (ND == 4 && NC == 3) dense = dense && n <= 704;
+      if (ND == 2 && NC == 2) dense = dense && n > 352;
     }
     auto run = [&](auto dp, auto ap) {
       ms_launch(w, st, dp, tile, dim3(128), w.g->geom, w.hgs, w.pb, w.w, w.G, w.kappa, w.grp, w.partials,
