@@ -105,3 +105,43 @@ def test_operators_and_observables_of_flagged_tensors(cuda_device, form):
     for rhs_per_thread in (0, 1):
         solver = dirac_solver.conjugate_gradient(tol=1e-10, rhs_per_thread=rhs_per_thread)
         assert torch.equal(solver.solve(op, form(b)), solver.solve(op, b))
+
+
+@pytest.mark.parametrize("geom,nc", [((5, 7), 2), ((3, 5, 2), 3), ((4, 3, 2, 5), 3), ((4, 3, 2, 5), 2)])
+def test_updates_in_place(cuda_device, geom, nc):
+    """The entry points a host calls on its own fields, and those whose output may be their input:
+    the bits of the call into another buffer."""
+    from tfleonardym_b200 import _dev, _lib, gauge_action, hmc
+    from tfleonardym_b200 import lattice as lt
+    rng = np.random.default_rng(int(np.prod(geom)))
+    nd, vol, L = len(geom), int(np.prod(geom)), _lib.lib()
+    u, p, f = cu(smooth_links(rng, geom, nc)), cu(momenta(rng, geom, nc)), cu(momenta(rng, geom, nc))
+    lat, st = lt.get_lattice(geom).handle, _dev.stream()
+    for reunitarize in (0, 1):
+        want = hmc.update_link_field(u, p, 0.1, reunitarize=bool(reunitarize))
+        for entry in ("update", "drift"):
+            x = u.clone()
+            if entry == "update":
+                rc = L.lym_update_links(nd, nc, vol, _dev.ptr(x), _dev.ptr(p), 0.1, reunitarize, st)
+            else:
+                rc = L.lym_link_drift(nd, nc, vol, _dev.ptr(x), _dev.ptr(p), 0.1, reunitarize, _dev.ptr(x), st)
+            assert rc == 0 and torch.equal(x, want), (entry, reunitarize)
+    want = hmc.update_momenta(p, f, 0.3)
+    for entry in ("update", "kick"):
+        x = p.clone()
+        if entry == "update":
+            rc = L.lym_update_momenta(p.numel(), _dev.ptr(x), _dev.ptr(f), 0.3, st)
+        else:
+            rc = L.lym_momenta_kick(p.numel(), _dev.ptr(x), _dev.ptr(f), 0.3, _dev.ptr(x), st)
+        assert rc == 0 and torch.equal(x, want), entry
+    action = gauge_action.yang_mills(lt.Configuration(u, geom, nc, nd), 5.5)
+    want = action.kicked_momenta(p, 0.2)
+    x = p.clone()
+    assert action.force_into_momenta(x, 0.2) is x and torch.equal(x, want)
+    x = p.clone()
+    assert L.lym_gauge_kick(lat, nc, 5.5, _dev.ptr(u), _dev.ptr(x), 0.2, _dev.ptr(x), st) == 0
+    assert torch.equal(x, want)
+    p_want, u_want = action.kick_and_drift(p, 0.2, 0.1)
+    x, y = p.clone(), torch.empty_like(u)
+    assert L.lym_gauge_kick_drift(lat, nc, 5.5, _dev.ptr(u), _dev.ptr(x), 0.2, 0.1, _dev.ptr(x), _dev.ptr(y), st) == 0
+    assert torch.equal(x, p_want) and torch.equal(y, u_want)

@@ -218,6 +218,123 @@ def test_hop_alone_after_a_one_launch_solve(cuda_device):
         assert _lib.lib().lym_dslash_eo(handle, _lib.PREC[precision], 999, 1, _dev.stream()) == _lib.LYM_ERR_BAD_ARG
 
 
+@pytest.mark.parametrize("precision", ["f64", "f32", "f16", "bf16"])
+@pytest.mark.parametrize("geoms,nc,herm", [([(8, 8), (4, 6), (32, 34)], 2, False), ([(6, 10), (12, 16)], 3, True),
+                                           ([(4, 4, 4, 4), (2, 4, 6, 8), (4, 4, 4, 10)], 3, False),
+                                           ([(4, 4, 4, 4), (2, 6, 4, 8)], 2, True),
+                                           ([(4, 4, 4), (8, 6, 4)], 3, False), ([(6, 4, 4), (16, 16, 16)], 2, False)])
+def test_lattices_launch_by_launch(cuda_device, geoms, nc, herm, precision):
+    """The kernels over all lattices of a call, which lists of small lattices reach only with a
+    forced tile: FP32 with the compressed links of SU(N) fields, FP16 with the mixed-precision hop
+    (2 and 4 dimensions).  The one-launch form solves the same systems."""
+    rng = np.random.default_rng(len(geoms) + nc)
+    systems = [System(rng, g, nc, 0.10 + 0.01 * k, herm) for k, g in enumerate(geoms)]
+    bs = [s.sources(rng, 1 + 2 * k) for k, s in enumerate(systems)]
+    for tiled in (1, 0, 1):
+        xs = [torch.empty_like(cu(b)) for b in bs]
+        rc, reps = solve_on(systems, [cu(b) for b in bs], xs, precision, rhs_per_thread=tiled)
+        assert rc == 0 and one_launch(reps) == (not tiled)
+        assert {r.compressed_links for r in reps} == {int(tiled and precision == "f32")}
+        assert {r.mixed_fma for r in reps} == {int(tiled and precision == "f16" and len(geoms[0]) != 3)}
+        for s, b, x in zip(systems, bs, xs):
+            assert max(s.residual(x[i], b[i]) for i in range(len(b))) < TOL
+
+
+@pytest.mark.parametrize("precision", ["f64", "f32", "f16"])
+def test_one_workspace_in_both_forms(cuda_device, precision):
+    """A workspace that the one-launch form left with more sources than a launch-by-launch solve
+    has: the padding starts empty again, so the solve takes the launches and gives the bits of one
+    on fresh links."""
+    rng = np.random.default_rng(12)
+    s = System(rng, (4, 4, 4, 8), 3)
+    b = cu(s.sources(rng, 8))
+
+    def solve(system, n, tiled):
+        x = torch.empty_like(b[:n])
+        rc, reps = solve_on([system], [b[:n]], [x], precision, rhs_per_thread=tiled)
+        assert rc == 0 and one_launch(reps) == (not tiled)
+        return x, reps[0].kernel_launches
+
+    for n, tiled in ((8, 0), (5, 1), (7, 0), (6, 1), (8, 1), (5, 0), (5, 1), (3, 0), (4, 0), (3, 1)):
+        x, launches = solve(s, n, tiled)
+        fresh = System.__new__(System)
+        fresh.__dict__.update(s.__dict__)
+        fresh.op = make_op(s.u, s.geom, s.kappa, False, "fundamental")
+        y, fresh_launches = solve(fresh, n, tiled)
+        assert torch.equal(x, y) and launches == fresh_launches, (n, tiled)
+        assert max(s.residual(x[i], b[i].cpu().numpy()) for i in range(n)) < TOL
+
+
+@pytest.mark.parametrize("geom,nc", [((4, 4, 4, 8), 3), ((4, 2, 4, 6), 2), ((8, 12), 3), ((4, 6, 4), 3)])
+@pytest.mark.parametrize("precision", ["f32", "f16", "bf16"])
+def test_compressed_links(cuda_device, geom, nc, precision):
+    rng = np.random.default_rng(nc)
+    s = System(rng, geom, nc)
+    b = s.sources(rng, 4)
+    for tile in (1, 2, 4):
+        x = torch.empty_like(cu(b))
+        rc, reps = solve_on([s], [cu(b)], [x], precision, rhs_per_thread=tile, compressed_links=1)
+        assert rc == 0 and {(r.rhs_per_thread, r.compressed_links) for r in reps} == {(tile, 1)}
+        assert max(s.residual(x[i], b[i]) for i in range(4)) < TOL
+
+
+# the sizes on either side of the one-launch rule, by its tables; 4D SU(3) FP64 takes 12 right-hand sides
+# up to 2048 sites per parity
+@pytest.mark.parametrize("geom,nc,precision,nrhs,resident",
+                         [((64, 128), 2, "f64", 1, True), ((64, 130), 2, "f64", 1, False),
+                          ((128, 128), 3, "f32", 2, True), ((128, 130), 3, "f32", 2, False),
+                          ((16, 16, 16), 3, "f64", 1, True), ((16, 16, 18), 3, "f64", 1, False),
+                          ((16, 16, 18), 3, "f16", 1, True), ((8, 8, 8, 8), 2, "f64", 12, True),
+                          ((8, 8, 8, 8), 2, "f64", 13, False), ((8, 8, 12, 16), 3, "f32", 3, False),
+                          ((8, 8, 12, 16), 2, "bf16", 2, False), ((8, 8, 8, 8), 3, "f16", 25, False)])
+def test_the_form_the_rule_takes(cuda_device, geom, nc, precision, nrhs, resident):
+    """Which form runs, and its answer; where it is not the resident one, with the tile that the
+    autotuner picks (compressed links among the FP32 and BF16 candidates)."""
+    rng = np.random.default_rng(int(np.prod(geom)))
+    s = System(rng, geom, nc)
+    b = s.sources(rng, nrhs)
+    x = torch.empty_like(cu(b))
+    rc, reps = solve_on([s], [cu(b)], [x], precision)
+    assert rc == 0 and one_launch(reps) == resident
+    for i in {0, nrhs // 2, nrhs - 1}:
+        assert s.residual(x[i], b[i]) < TOL
+
+
+# more than 64 MB of links in the precision of the hop and several tiles: the right-hand side is the
+# fast index of the grid (in every hop of the FP64 solve, in the FP64 updates of the others, in the sloppy
+# hops from 24^3 x 16 in FP32 and 24^3 x 32 in FP16 on); 16^3 x 28 lies below in FP64
+@pytest.mark.parametrize("geom,nc,precision,nrhs,tile", [((16, 16, 16, 28), 3, "f64", 2, 0),
+                                                         ((16, 16, 16, 32), 3, "f64", 2, 0),
+                                                         ((16, 16, 16, 30), 3, "f64", 3, 0),
+                                                         ((16, 16, 16, 32), 3, "f32", 4, 2),
+                                                         ((24, 24, 24, 16), 3, "f32", 4, 2),
+                                                         ((24, 24, 24, 16), 3, "f32", 8, 4),
+                                                         ((24, 24, 24, 32), 3, "f16", 4, 1),
+                                                         ((24, 24, 24, 32), 3, "f16", 4, 0)])
+def test_grids_with_the_right_hand_side_fastest(cuda_device, geom, nc, precision, nrhs, tile):
+    s = LargeSystem(geom, nc)
+    b = s.normal((nrhs,) + s.shape)
+    b *= torch.arange(1, nrhs + 1, device="cuda")[:, None, None, None]  # sources that cannot be taken for each other
+    x = torch.empty_like(b)
+    rc, reps = solve_on([s], [b], [x], precision, rhs_per_thread=tile)
+    assert rc == 0 and (not tile or reps[0].rhs_per_thread == tile)
+    assert max(s.residual(x[i], b[i]) for i in range(nrhs)) < TOL
+
+
+@pytest.mark.parametrize("geom,nc,precision,nrhs", [((16, 16, 16), 2, "f64", 40), ((16, 16, 16), 2, "f32", 64),
+                                                    ((32, 66), 3, "f64", 64), ((32, 66), 3, "f16", 40),
+                                                    ((8, 8, 8, 8), 3, "f32", 24)])
+def test_more_clusters_than_fit_at_once(cuda_device, geom, nc, precision, nrhs):
+    """Above 1024 sites per parity with more right-hand sides than clusters of 8 x 256 threads fit:
+    clusters of 8 x 128."""
+    s = LargeSystem(geom, nc)
+    b = s.normal((nrhs,) + s.shape)
+    x = torch.empty_like(b)
+    rc, reps = solve_on([s], [b], [x], precision)
+    assert rc == 0 and one_launch(reps)
+    assert max(s.residual(x[i], b[i]) for i in range(nrhs)) < TOL
+
+
 # blocks of the operator kernels: 324 and 392 (one wave of three per SM instead of two of two) and 640 (two
 # instead of three); the usual form for 314 in 2D SU(2), 768 in 4D SU(3) and 512
 @pytest.mark.parametrize("geom,nc", [((12, 12, 12, 24), 3), ((12, 12, 12, 24), 2), ((224, 224), 2), ((200, 200), 2),
