@@ -1,0 +1,69 @@
+"""Rounding of the gauge and force kernels against extended precision (80-bit, so that the
+reference's own rounding, which is the kernels' in 64 bits, does not count).
+
+Bounds, relative in the 2-norm: what the plainest evaluation gives -- every product formed by itself,
+then added -- and 5 % for the draw of the inputs.  Products that accumulate into a long sum lie 20 to
+35 % above, short-cut angles 6 %.
+"""
+import numpy as np
+import pytest
+import torch
+
+from oracle import lym_oracle as O
+from tests.test_gpu_kernel_edges import cnormal, cu, smooth_links
+
+pytestmark = pytest.mark.gpu
+
+L, CL = np.longdouble, np.clongdouble
+
+
+def mm(a, b):
+    return np.einsum("ijv,jkv->ikv", a, b)
+
+
+def dag(a):
+    return np.conj(np.swapaxes(a, 0, 1))
+
+
+def off(got, exact):
+    got = got.cpu().numpy() if isinstance(got, torch.Tensor) else got
+    return float(np.sqrt(np.sum(np.abs(got - exact) ** 2) / np.sum(np.abs(exact) ** 2)))
+
+
+def momenta(rng, geom, nc):
+    x = 0.5 * cnormal(rng, (len(geom), nc, nc, int(np.prod(geom))))
+    p = x - np.conj(np.swapaxes(x, 1, 2))
+    return p - np.einsum("miiv->mv", p)[:, None, None] * (np.eye(nc) / nc)[None, :, :, None]
+
+
+def configuration(u, geom):
+    from tfleonardym_b200 import lattice as lt
+    return lt.Configuration(cu(u), geom, u.shape[1], len(geom))
+
+
+# plainest: 1.14e-16 and 1.35e-16
+@pytest.mark.parametrize("nc,bound", [(2, 1.2e-16), (3, 1.42e-16)])
+def test_gauge_force(cuda_device, nc, bound):
+    from tfleonardym_b200 import gauge_action, staples
+    geom, beta = (6, 6, 6, 8), 5.5
+    rng = np.random.default_rng(nc)
+    u, tables = smooth_links(rng, geom, nc, spread=0.25), O.lookup_tables(geom)
+    x = u.astype(CL)
+    exact, sums = [], []
+    for mu in range(4):
+        s = np.zeros(x.shape[1:], CL)
+        for nu in range(4):
+            if nu != mu:
+                s += mm(mm(x[nu], O.translate(x[mu], tables, nu, 1)), dag(O.translate(x[nu], tables, mu, 1)))
+                s += O.translate(mm(mm(dag(x[nu]), x[mu]), O.translate(x[nu], tables, mu, 1)), tables, nu, -1)
+        w = mm(x[mu], dag(s))
+        f = -L(beta) / (4 * nc) * (dag(w) - w)
+        sums.append(s)
+        exact.append(f - np.einsum("iiv->v", f) / nc * np.eye(nc)[:, :, None])
+    action = gauge_action.yang_mills(configuration(u, geom), beta)
+    assert off(action.force(), np.stack(exact)) < bound
+    assert off(staples.get_staple_sums(action.cfg, -1), np.stack(sums)) < bound
+    p = momenta(rng, geom, nc)
+    kicked = action.kicked_momenta(cu(p), 1.0).cpu().numpy()
+    assert off(kicked, p.astype(CL) + np.stack(exact)) < bound
+    assert np.array_equal(action.kick_and_drift(cu(p), 1.0, 0.1)[0].cpu().numpy(), kicked)

@@ -21,19 +21,25 @@ namespace lym {
 
 // Row by row, so that only two neighbour links and one row are live beside the sum
 // (168 registers at three blocks per SM, 128 at four, where whole products took 184 and
-// left two) and the second product accumulates into the sum with fused multiply-adds.
-// Bound by the latency of its gathers: at 16^3 x 32 SU(3) the force kernel takes 100 us
-// against 150 us before (FP64 pipe 47 %, L1 52 % busy; the FP64 work alone is 45 us); the
-// staples alone at 24^3 x 48 258 us against 361 us (four blocks; 281 us with three, which
-// the force, with its larger tail, runs as fast).
-template <int ND, int NC>
+// left two).  Bound by the latency of its gathers: at 16^3 x 32 SU(3) the force kernel takes
+// 101 us against 150 us with whole products (blocks of 128; FP64 pipe 47 %, L1 52 % busy;
+// the FP64 work alone is 45 us), the staples alone at 24^3 x 48 258 us against 361 us.
+// FUSED: the second product accumulates straight into the sum, 36 roundings of it in 4D.
+// Otherwise each staple is formed by itself and added once, six roundings: the force is
+// 1.39e-16 off 64-bit-exact values (2-norm, SU(3)) and 1.80e-16 with FUSED, whole products
+// 1.35e-16; FUSED serves smearing alone, whose projection outweighs it (1.1e-16 either way)
+// and whose registers it saves (3 %).
+// The planes one after the other: with all loads of a link free to move, ptxas gathers more of
+// them ahead than the registers hold (the force in blocks of 256 spills 400 bytes and takes 20 %
+// longer).  A rolled loop does it in blocks of 128 for SU(3) (2 to 5 % faster than the
+// unrolled one), a pointer that depends on the sum so far does it in the others (rolled:
+// 12 % slower in blocks of 256).
+template <int ND, int NC, bool FUSED, bool ROLLED>
 LYM_D Mat<NC> staple_sum(const int32_t* __restrict__ tab, int64_t V, const double2* __restrict__ U, int mu,
                          int64_t s, int no_dir) {
   Mat<NC> S = mzero<NC>();
   const int64_t xmu = tab[mu * V + s];
-#pragma unroll
-  for (int nu = 0; nu < ND; ++nu) {
-    if (nu == mu || nu == no_dir) continue;
+  auto plane = [&](int nu) {
     const int64_t xnu = tab[nu * V + s];
     const int64_t xmnu = tab[ND * V + nu * V + s];
     const int64_t xmnu_pmu = tab[mu * V + xmnu];
@@ -45,7 +51,17 @@ LYM_D Mat<NC> staple_sum(const int32_t* __restrict__ tab, int64_t V, const doubl
 #pragma unroll
         for (int k = 0; k < NC; ++k) a[k] = ld(U + ((int64_t)(nu * NC + i) * NC + k) * V + s);
         row_mul<NC>(r, a, b);
-        row_mac_nd<NC>(S.m[i], r, c);
+        if constexpr (FUSED) {
+          row_mac_nd<NC>(S.m[i], r, c);
+        } else {
+#pragma unroll
+          for (int j = 0; j < NC; ++j) {
+            cx<double> t = cmul_cj(c.m[j][0], r[0]);
+#pragma unroll
+            for (int k = 1; k < NC; ++k) cmac_cj(t, c.m[j][k], r[k]);
+            S.m[i][j] += t;
+          }
+        }
       }
     }
     {
@@ -56,8 +72,32 @@ LYM_D Mat<NC> staple_sum(const int32_t* __restrict__ tab, int64_t V, const doubl
 #pragma unroll
         for (int k = 0; k < NC; ++k) a[k] = conj(ld(U + ((int64_t)(nu * NC + k) * NC + i) * V + xmnu));
         row_mul<NC>(r, a, b);
-        row_mac<NC>(S.m[i], r, c);
+        if constexpr (FUSED) {
+          row_mac<NC>(S.m[i], r, c);
+        } else {
+#pragma unroll
+          for (int j = 0; j < NC; ++j) {
+            cx<double> t = r[0] * c.m[0][j];
+#pragma unroll
+            for (int k = 1; k < NC; ++k) cmac(t, r[k], c.m[k][j]);
+            S.m[i][j] += t;
+          }
+        }
       }
+    }
+  };
+  if constexpr (ROLLED) {
+#pragma unroll 1
+    for (int p = 0; p < ND - 1; ++p) {
+      const int nu = p + (p >= mu ? 1 : 0);
+      if (nu != no_dir) plane(nu);
+    }
+  } else {
+#pragma unroll
+    for (int nu = 0; nu < ND; ++nu) {
+      if (nu == mu || nu == no_dir) continue;
+      if constexpr (!FUSED) asm volatile("" : "+l"(U) : "d"(S.m[0][0].re), "d"(S.m[NC - 1][NC - 1].im));
+      plane(nu);
     }
   }
   return S;
@@ -70,7 +110,7 @@ __global__ void __launch_bounds__(128, 4) staples_kernel(const int32_t* __restri
   int mu;
   int64_t s;
   if (!warp_link(ND, V, blockIdx.x, mu, s)) return;
-  Mat<NC> S = (mu == no_dir) ? mzero<NC>() : staple_sum<ND, NC>(tab, V, U, mu, s, no_dir);
+  Mat<NC> S = (mu == no_dir) ? mzero<NC>() : staple_sum<ND, NC, false, NC == 3>(tab, V, U, mu, s, no_dir);
   store_link<NC>(out, mu, s, V, S);
 }
 
@@ -107,22 +147,39 @@ __global__ void __launch_bounds__(128) staple_terms_kernel(const int32_t* __rest
   }
 }
 
-// F = -beta/(4N) (W^dag - W) - trace/N, W = U S^dag at one link (gauge_action.py:42-53)
-template <int ND, int NC>
+// F = -beta/(4N) (W^dag - W) - trace/N, W = U S^dag at one link (gauge_action.py:42-53);
+// anti-Hermitian, so the upper triangle of W^dag - W gives the lower one
+template <int ND, int NC, bool ROLLED>
 LYM_D Mat<NC> gauge_force_link(const int32_t* __restrict__ tab, int64_t V, const double2* __restrict__ U,
                                double beta, int mu, int64_t s) {
-  Mat<NC> S = staple_sum<ND, NC>(tab, V, U, mu, s, -1);
-  Mat<NC> W = mul_nd(load_link<NC>(U, mu, s, V), S);
+  const Mat<NC> S = staple_sum<ND, NC, false, ROLLED>(tab, V, U, mu, s, -1);
+  // the link's loads after the staples: ahead of them they would only hold registers
+  asm volatile("" : "+l"(U) : "d"(S.m[0][0].re), "d"(S.m[NC - 1][NC - 1].im));
+  const Mat<NC> L = load_link<NC>(U, mu, s, V);
   const double c = -0.25 * beta / NC;
   Mat<NC> F;
+  double tr = 0.0;
 #pragma unroll
-  for (int i = 0; i < NC; ++i)
+  for (int i = 0; i < NC; ++i) {
+    cx<double> w = cmul_cj(S.m[i][0], L.m[i][0]);
 #pragma unroll
-    for (int j = 0; j < NC; ++j) F.m[i][j] = c * (conj(W.m[j][i]) - W.m[i][j]);
-  cx<double> tr = trace(F);
-  tr = (1.0 / NC) * tr;
+    for (int k = 1; k < NC; ++k) cmac_cj(w, S.m[i][k], L.m[i][k]);
+    F.m[i][i] = {0.0, c * (-w.im - w.im)};
+    tr += F.m[i][i].im;
 #pragma unroll
-  for (int i = 0; i < NC; ++i) F.m[i][i] -= tr;
+    for (int j = i + 1; j < NC; ++j) {
+      cx<double> x = cmul_cj(S.m[j][0], L.m[i][0]), y = cmul_cj(S.m[i][0], L.m[j][0]);
+#pragma unroll
+      for (int k = 1; k < NC; ++k) {
+        cmac_cj(x, S.m[j][k], L.m[i][k]);
+        cmac_cj(y, S.m[i][k], L.m[j][k]);
+      }
+      F.m[i][j] = c * (conj(y) - x);
+      F.m[j][i] = -conj(F.m[i][j]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NC; ++i) F.m[i][i].im -= (1.0 / NC) * tr;
   return F;
 }
 
@@ -136,7 +193,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 256 ? 2 : NC == 2 ? 4 : 3)
   int mu;
   int64_t s;
   if (!warp_link(ND, V, blockIdx.x, mu, s)) return;
-  Mat<NC> F = gauge_force_link<ND, NC>(tab, V, U, beta, mu, s);
+  Mat<NC> F = gauge_force_link<ND, NC, NC == 3 && BLOCK == 128>(tab, V, U, beta, mu, s);
   if (mom) {
     Mat<NC> P;  // all of it before the first store: out may be mom
 #pragma unroll
@@ -602,7 +659,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 256 ? 2 : 4)
   if (mu == no_dir) {
     F = mscale(rho, load_link<NC>(U, mu, s, V));
   } else {
-    F = mscale(cx<double>{rho.re / 6, rho.im / 6}, staple_sum<ND, NC>(tab, V, U, mu, s, no_dir));
+    F = mscale(cx<double>{rho.re / 6, rho.im / 6}, staple_sum<ND, NC, true, false>(tab, V, U, mu, s, no_dir));
   }
 #pragma unroll
   for (int i = 0; i < NC; ++i)
@@ -725,7 +782,7 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 256 ? 2 : NC == 2 ? 4 : 3)
   int mu;
   int64_t s;
   if (!warp_link(ND, V, blockIdx.x, mu, s)) return;
-  const Mat<NC> F = gauge_force_link<ND, NC>(tab, V, U, beta, mu, s);
+  const Mat<NC> F = gauge_force_link<ND, NC, NC == 3 && BLOCK == 128>(tab, V, U, beta, mu, s);
   Mat<NC> P;  // all of it before the first store: mom_out may be mom
 #pragma unroll
   for (int k = 0; k < NC * NC; ++k) {
@@ -777,7 +834,7 @@ LYM_D int hmc_lat_of(const HmcTable& t, int b) {
 
 template <int ND, int NC>
 LYM_D void hmc_kick_link(const HmcLat& L, double eps, int mu, int64_t s) {
-  const Mat<NC> F = gauge_force_link<ND, NC>(L.tab, L.V, L.U, L.beta, mu, s);
+  const Mat<NC> F = gauge_force_link<ND, NC, NC == 3>(L.tab, L.V, L.U, L.beta, mu, s);
   Mat<NC> P = load_link<NC>(L.P, mu, s, L.V);
 #pragma unroll
   for (int i = 0; i < NC; ++i)
