@@ -681,10 +681,12 @@ __global__ void __launch_bounds__(BLOCK, BLOCK == 256 ? 2 : 4)
 //   hermitian:  A = sum_a conj(x+) (x) v-,   B = A^dag (one outer product per row)
 //   plain:      A = sum_a conj(x-) (x) v-,   B = sum_a conj(v+) (x) x+
 // so a link and pole costs ns/2 matvecs and outer products per ordering instead of ns
-// matvecs, two full projections and 2 ns outer products, which spilled; the poles'
-// weights go into the sum.  12^3 x 24 SU(3), 8 poles: 97 us against 336 us, 16^4, 10 poles: 172 us
-// against 620 us (three blocks per SM; two take 180, four spill and take 186); bound by
-// the four spinor gathers per link and pole.
+// matvecs, two full projections and 2 ns outer products, which spilled.  Each pole's terms are
+// summed by themselves and added with its weight: straight into the sum, every product is rounded
+// against all poles before it (SU(3), 4 poles: 2.4e-16 off exact values instead of 1.8e-16).  The sum
+// waits in shared memory, where registers would spill.  12^3 x 24 SU(3), 8 poles: 95 us against
+// 336 us, 16^4, 10 poles: 174 us against 620 us (three blocks per SM); bound by the four spinor
+// gathers per link and pole.
 // ---------------------------------------------------------------------------
 constexpr int kMaxForceTerms = 64;
 struct ForceTerms {
@@ -718,10 +720,14 @@ __global__ void __launch_bounds__(128, 3) fermion_force_kernel(
   const int64_t y = tab[mu * V + s];
   Mat<NC> u = load_link<NC>(U, mu, s, V);
   if (mu == ND - 1 && (s % Lt) == Lt - 1) u = mscale(cx<double>{bcr, bci}, u);
-  Mat<NC> K = mzero<NC>();  // sum over the poles of w (A - B), hermitian: of w A
+  __shared__ double2 sum[NC * NC][128];  // over the poles: w (A - B), hermitian: w A
+#pragma unroll
+  for (int i = 0; i < NC * NC; ++i) sum[i][threadIdx.x] = make_double2(0.0, 0.0);
+  Mat<NC> K;
   const int64_t vec = (int64_t)NS * NC * V;
   for (int k = 0; k < nterms; ++k) {
     const double w = 0.5 * kappa * terms.alpha[k];
+    K = mzero<NC>();
     for (int side = 0; side < (symmetric ? 2 : 1); ++side) {
       const double2* P = (side == 0 ? X : Y) + k * vec;  // L(P, Q): P at x, Q at x + mu
       const double2* Q = (side == 0 ? Y : X) + k * vec;
@@ -732,13 +738,12 @@ __global__ void __launch_bounds__(128, 3) fermion_force_kernel(
         cx<double> h[NC], q[NC];
         half_row<ND, NC>(P, mu, a, HERM || plus, V, s, h);
         half_row<ND, NC>(Q, mu, a, plus, V, y, q);
-        const double wc = plus ? -w : w;
 #pragma unroll
         for (int i = 0; i < NC; ++i) {
           cx<double> v = u.m[i][0] * q[0];
 #pragma unroll
           for (int l = 1; l < NC; ++l) cmac(v, u.m[i][l], q[l]);
-          v = wc * v;
+          if (plus) v = -v;
 #pragma unroll
           for (int j = 0; j < NC; ++j) {
             if (plus) cmac_cj(K.m[i][j], v, h[j]);  // conj(v)_i x_j
@@ -747,7 +752,15 @@ __global__ void __launch_bounds__(128, 3) fermion_force_kernel(
         }
       }
     }
+#pragma unroll
+    for (int i = 0; i < NC * NC; ++i) {
+      double2& o = sum[i][threadIdx.x];
+      const cx<double> t = K.m[i / NC][i % NC];
+      o = make_double2(fma(w, t.re, o.x), fma(w, t.im, o.y));
+    }
   }
+#pragma unroll
+  for (int i = 0; i < NC * NC; ++i) K.m[i / NC][i % NC] = {sum[i][threadIdx.x].x, sum[i][threadIdx.x].y};
   if constexpr (HERM) {
     Mat<NC> D;
 #pragma unroll
