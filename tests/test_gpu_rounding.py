@@ -97,3 +97,21 @@ def test_fundamental_force_of_several_poles(cuda_device, nc, geom):
                                    boundary_condition_provider=bc.time_antiperiodic_provider(-1))
     force = op.accumulate_force(torch.zeros_like(op.cfg.gauge_field), alphas, cu(x), cu(y), symmetric=True)
     assert off(force, np.stack(exact)) < 1.96e-16
+
+
+# plainest: 1.47e-16
+@pytest.mark.parametrize("eps", [0.01, 0.1])
+def test_drift(cuda_device, eps):
+    from tfleonardym_b200 import hmc
+    geom, nc = (6, 6, 6, 8), 3
+    rng = np.random.default_rng(5)
+    u, p = smooth_links(rng, geom, nc, spread=0.25), momenta(rng, geom, nc)
+    exact = []
+    for mu in range(4):
+        x = p[mu].astype(CL) * L(eps)
+        term = total = np.broadcast_to(np.eye(nc, dtype=CL)[:, :, None], x.shape)
+        for k in range(1, 40):
+            term = mm(term, x) / k
+            total = total + term
+        exact.append(mm(total, u[mu].astype(CL)))
+    assert off(hmc.update_link_field(cu(u), cu(p), eps), np.stack(exact)) < 1.54e-16

@@ -409,8 +409,8 @@ LYM_D Mat<3> expm(const Mat<3>& X) {
     const double u2 = u * u, w2 = w * w;
     double s2u, c2u, su, cu;
     sincos(u, &su, &cu);
-    s2u = 2.0 * su * cu;
-    c2u = (cu - su) * (cu + su);
+    // by itself: from su and cu the drift is 1.55e-16 off exact values instead of 1.45e-16
+    sincos(2.0 * u, &s2u, &c2u);
     const cx<double> e2iu{c2u, s2u}, emiu{cu, -su};
     const double cw = cos(w), xi0 = sinc(w);
     cx<double> h0 = (u2 - w2) * e2iu + emiu * cx<double>{8.0 * u2 * cw, 2.0 * u * (3.0 * u2 + w2) * xi0};
