@@ -115,3 +115,23 @@ def test_drift(cuda_device, eps):
             total = total + term
         exact.append(mm(total, u[mu].astype(CL)))
     assert off(hmc.update_link_field(cu(u), cu(p), eps), np.stack(exact)) < 1.54e-16
+
+
+# plainest: 1.08e-16
+def test_traces_of_four_links(cuda_device):
+    from tfleonardym_b200 import _dev, _lib, measurements
+    geom, nc, bound = (6, 6, 6, 8), 3, 1.13e-16
+    rng = np.random.default_rng(nc)
+    u, tables = smooth_links(rng, geom, nc, spread=0.25), O.lookup_tables(geom)
+    x, cfg = u.astype(CL), configuration(u, geom)
+    total = 0
+    for a in range(4):
+        for b in range(a + 1, 4):
+            loop = mm(mm(x[a], O.translate(x[b], tables, a, 1)), dag(mm(x[b], O.translate(x[a], tables, b, 1))))
+            trace = np.einsum("iiv->v", loop)
+            assert off(measurements.path_field(cfg, [a + 1, b + 1, -a - 1, -b - 1]), trace) < bound, (a, b)
+            total = total + trace
+    plaquettes, squares = (torch.empty(u.shape[-1], dtype=torch.complex128, device="cuda") for _ in range(2))
+    _lib.check(_lib.lib().lym_plane_loops(measurements._lattice(cfg).handle, nc, _dev.ptr(cfg.gauge_field), -1,
+                                          _dev.ptr(plaquettes), _dev.ptr(squares), _dev.stream()), "lym_plane_loops")
+    assert off(plaquettes, total) < bound

@@ -1213,12 +1213,15 @@ __global__ void __launch_bounds__(128) path_kernel(const int32_t* __restrict__ t
     } else if (want_trace && k == nsteps - 1) {
       cx<double> t = czero<double>();
 #pragma unroll
-      for (int i = 0; i < NC; ++i)
+      for (int i = 0; i < NC; ++i) {  // a diagonal element by itself: the trace is rounded N times, not 2 N^2
+        cx<double> d = s > 0 ? m.m[i][0] * l.m[0][i] : cmul_cj(l.m[i][0], m.m[i][0]);
 #pragma unroll
-        for (int j = 0; j < NC; ++j) {
-          if (s > 0) cmac(t, m.m[i][j], l.m[j][i]);
-          else cmac_cj(t, l.m[i][j], m.m[i][j]);
+        for (int j = 1; j < NC; ++j) {
+          if (s > 0) cmac(d, m.m[i][j], l.m[j][i]);
+          else cmac_cj(d, l.m[i][j], m.m[i][j]);
         }
+        t += d;
+      }
       st(out + x, t);
       return;
     } else if (s > 0) {
@@ -1235,6 +1238,15 @@ __global__ void __launch_bounds__(128) path_kernel(const int32_t* __restrict__ t
 #pragma unroll
       for (int j = 0; j < NC; ++j) st(out + ((int64_t)i * NC + j) * V + x, m.m[i][j]);
   }
+}
+
+// t += conj(r) . q, the product of the rows formed by itself
+template <int NC>
+LYM_D void add_dot(cx<double>& t, const cx<double> (&r)[NC], const cx<double> (&q)[NC]) {
+  cx<double> d = cmul_cj(r[0], q[0]);
+#pragma unroll
+  for (int k = 1; k < NC; ++k) cmac_cj(d, r[k], q[k]);
+  t += d;
 }
 
 // plaq(x), square(x) = sum over the planes without direction `skip` of the traces of the
@@ -1256,6 +1268,7 @@ __global__ void __launch_bounds__(128, 3) plane_loops_kernel(const int32_t* __re
       if (a == skip || b == skip) continue;
       const int64_t xa = tab[a * V + x], xb = tab[b * V + x], xaa = tab[a * V + xa], xbb = tab[b * V + xb];
       const int64_t xaab = tab[b * V + xaa], xbba = tab[a * V + xbb];
+      cx<double> loop = czero<double>();
       {
         const Mat<NC> b1 = load_link<NC>(U, b, xa, V), c1 = load_link<NC>(U, a, xb, V);
 #pragma unroll
@@ -1267,10 +1280,11 @@ __global__ void __launch_bounds__(128, 3) plane_loops_kernel(const int32_t* __re
 #pragma unroll
           for (int k = 0; k < NC; ++k) p[k] = ld(U + ((int64_t)(b * NC + i) * NC + k) * V + x);
           row_mul<NC>(r, p, c1);
-#pragma unroll
-          for (int k = 0; k < NC; ++k) cmac_cj(tp, r[k], q[k]);
+          add_dot<NC>(loop, r, q);
         }
       }
+      tp += loop;
+      loop = czero<double>();
       Mat<NC> p = mul(load_link<NC>(U, a, x, V), load_link<NC>(U, a, xa, V));
       p = mul(p, load_link<NC>(U, b, xaa, V));
       p = mul(p, load_link<NC>(U, b, xaab, V));
@@ -1281,9 +1295,9 @@ __global__ void __launch_bounds__(128, 3) plane_loops_kernel(const int32_t* __re
       for (int i = 0; i < NC; ++i) {
         cx<double> r[NC];
         row_mul<NC>(r, q.m[i], l);
-#pragma unroll
-        for (int k = 0; k < NC; ++k) cmac_cj(ts, r[k], p.m[i][k]);
+        add_dot<NC>(loop, r, p.m[i]);
       }
+      ts += loop;
     }
   st(plaq + x, tp);
   st(square + x, ts);
