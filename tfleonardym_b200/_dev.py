@@ -5,6 +5,8 @@ import torch
 
 from . import _lib
 
+_Tensor, _C128 = torch.Tensor, torch.complex128  # looked up once: as_c128 runs several times a call
+
 
 def require_cuda():
     if not torch.cuda.is_available():
@@ -20,12 +22,12 @@ def as_c128(t, name="tensor"):
 
     Its memory holds its values: a lazy conjugate or sign, which torch keeps as a flag that
     contiguous() passes on, is written out (into a copy; without a flag nothing is copied)."""
-    if not isinstance(t, torch.Tensor):
+    if not isinstance(t, _Tensor):
         t = torch.from_dlpack(t)
     if not t.is_cuda:
         raise ValueError(f"{name} must be a CUDA tensor")
-    if t.dtype != torch.complex128:
-        t = t.to(torch.complex128)
+    if t.dtype is not _C128:
+        t = t.to(_C128)
     t = t.contiguous()
     if t.is_conj() or t.is_neg():  # two flags to test cost half of what the two calls below do
         t = t.resolve_conj().resolve_neg()
