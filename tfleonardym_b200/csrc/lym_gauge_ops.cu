@@ -21,8 +21,8 @@ namespace lym {
 
 // Row by row, so that only two neighbour links and one row are live beside the sum
 // (168 registers at three blocks per SM, 128 at four, where whole products took 184 and
-// left two).  Bound by the latency of its gathers: at 16^3 x 32 SU(3) the force kernel takes
-// 101 us against 150 us with whole products (blocks of 128; FP64 pipe 47 %, L1 52 % busy;
+// left two).  Bound by the latency of its gathers: within a trajectory at 16^3 x 32 SU(3) the
+// force kernel takes 95 us against 150 us with whole products (FP64 pipe 47 %, L1 52 % busy;
 // the FP64 work alone is 45 us), the staples alone at 24^3 x 48 258 us against 361 us.
 // FUSED: the second product accumulates straight into the sum, 36 roundings of it in 4D.
 // Otherwise each staple is formed by itself and added once, six roundings: the force is
@@ -901,7 +901,7 @@ __global__ void __launch_bounds__(128) hmc_multi_kernel(const __grid_constant__ 
 // Link kernels whose 4D SU(3) form at 128 registers is worth blocks of eight warps: 64 sites
 // and their directions share an SM's L1, and the block's rows of loads go out together.  From
 // three waves of sixteen warps per SM on: force / kick and drift / smear in us with 256 | 128
-// threads, 16^3 x 32 85.3 / 128.0 / 106.1 | 90.0 / 141.4 / 121.5, 16^4 42.7 / 66.9 / 53.1 |
+// threads (launches in a row, random links), 16^3 x 32 85.3 / 128.0 / 106.1 | 90.0 / 141.4 / 121.5, 16^4 42.7 / 66.9 / 53.1 |
 // 45.3 / 72.8 / 61.1; below, 12^3 x 24 29.5 / 48.1 / 37.5 | 28.5 / 45.8 / 41.0, 8^4 7.9 / 11.7 /
 // 10.3 | 5.9 / 9.6 / 9.1.  SU(2) and fewer dimensions gain nothing (24^4 SU(2) 94.7 / 145.6 /
 // 146 | 92.4 / 142.1 / 140).
@@ -1252,7 +1252,7 @@ LYM_D void add_dot(cx<double>& t, const cx<double> (&r)[NC], const cx<double> (&
 // plaq(x), square(x) = sum over the planes without direction `skip` of the traces of the
 // 1 x 1 and 2 x 2 loops from x (measurements.py:197-290), each loop as its two halves
 // (Tr P Q^dag), all planes of a site in one thread: ten distinct links per plane, no
-// per-plane fields.  24^3 x 48 SU(3), three planes: 248 us against 1130 us for the six paths and
+// per-plane fields.  24^3 x 48 SU(3), three planes: 235 us against 1130 us for the six paths and
 // their sums.
 template <int NC>
 __global__ void __launch_bounds__(128, 3) plane_loops_kernel(const int32_t* __restrict__ tab, int nd, int64_t V,
@@ -1307,7 +1307,7 @@ __global__ void __launch_bounds__(128, 3) plane_loops_kernel(const int32_t* __re
 // the same from every site of a line, so a line is multiplied once -- kPolySeg threads
 // each take a segment -- and its trace written to all of its sites, where the general
 // path multiplies the line from each of its L_d sites.  24^3 x 48 SU(3), 48 links:
-// 31 us against 319 us.
+// 39 us against 319 us.
 constexpr int kPolySeg = 4;
 template <int NC>
 __global__ void __launch_bounds__(32 * kPolySeg) loop_kernel(int64_t nlines, int64_t V, int64_t stride, int L,
@@ -1349,7 +1349,7 @@ __global__ void __launch_bounds__(32 * kPolySeg) loop_kernel(int64_t nlines, int
 // out[2z], out[2z+1] = sum of f(x) over the sites with x_dir = z (and, when
 // mask_len > 0, x_mask = 0); x_d = (x / stride_d) mod L_d for the lexicographic
 // index with the last coordinate fastest.  The cluster walks its slice's sites only
-// (24^3 x 48: 5.4 us against 712 us for one block per slice that tested every site of
+// (24^3 x 48: 6 us against 712 us for one block per slice that tested every site of
 // the lattice).
 __global__ void __cluster_dims__(kSliceCtas, 1, 1) __launch_bounds__(kSliceThreads)
     slice_sum_kernel(uint32_t per, uint32_t stride, uint32_t L, uint32_t mask_stride, uint32_t mask_len,

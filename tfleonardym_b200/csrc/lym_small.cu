@@ -446,9 +446,14 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
 //     with 1 rhs and 2196 / 1903 with 16, 8^3 x 16 2440 / 1597
 //   FP32 (FP16):  2D 128^2 571 / 1550 (539 / 1208); 3D 24^3 887 / 1923 (821 / 1389); 4D SU(3)
 //     8^3 x 16 1971 / 3132 (1798 / 2407) with 1 rhs, 3435 / 4174 (3090 / 2983) with 16
+//   The other classes, time of the graph form over this one's with 1 / 12 / 32 rhs (-: above the
+//     rule): FP64 3D SU(3) 16^3 1.53 / 1.78 / 1.65, 4D SU(2) 8^4 1.47 / 1.68 / -, 2D SU(3) 64 x 128
+//     1.29 / 1.75 / 1.68; FP32 4.1 / 4.5 / 3.1, 3.3 / 3.3 / 2.4 and 3.2 / 3.5 / 2.8; 64 rhs 64 x 128 1.47,
+//     16^3 1.33 in FP64.
 //   several lattices, whose graph form copies state per lattice at every wait: faster at
 //     every size measured, 84 systems on 21 4D SU(3) lattices up to 1536 sites per parity
-//     4447 / 6023 us in FP64 and 3653 / 9415 in FP32
+//     4447 / 6023 us in FP64 and 3653 / 9415 in FP32; 1024 systems on 64 lattices 1.08 (FP64) and
+//     1.36 (FP32) times in 4D SU(3), 1.31 and 1.43 in 4D SU(2), 1.4 to 2.0 in 3D, 1.5 to 2.3 in 2D
 bool small_applies(int nd, int nc, int sp, int64_t vh, int systems, int lattices) {
   if (lattices > 1 && vh <= 2048) return systems <= 1024;
   if (systems > 64) return false;
