@@ -268,6 +268,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
     q2 = cluster_sum(cs, n);
   }
   const double want = L.tol * L.tol * bnorm2;
+  const int limit = min(L.max_iter, stop);
   while (true) {
     const bool fwd = mode == 0;
     for (int i = tid; i < vh; i += T) {
@@ -333,13 +334,13 @@ __global__ void __launch_bounds__(kSmallThreads, 1)
         store_sp<SP, NCOMP>(L.p, rhs, i, p);
       }
       cluster_sync(single);
-      if (!(rr < pause2 || iters >= L.max_iter || iters >= pause_iter)) {
-        if (iters >= stop) {
-          going = true;
-          break;
-        }
+      if (!(rr < pause2 || iters >= limit || iters >= pause_iter)) {
         mode = 0;
         continue;
+      }
+      if (!(rr < pause2 || iters >= L.max_iter || iters >= pause_iter)) {
+        going = true;
+        break;
       }
     } else {
       // the plan for the next run (the rules of cg_solve_on)
