@@ -14,7 +14,8 @@ def require_cuda():
 
 
 def stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    # the handle of torch.cuda.current_stream() without the object around it (0.3 us instead of 3.3)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
 
 
 def as_c128(t, name="tensor"):
