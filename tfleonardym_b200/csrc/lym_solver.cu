@@ -300,12 +300,12 @@ LYM_D void rhs_tile(const EoGeom& g, int& bx, int& by) {
 struct HopGrid {
   EoGeom g;
   dim3 grid;
-  // FP64 hop kernels in the form with three blocks per SM: beyond two waves of two, and for
-  // 4D SU(3) below nine waves only where it saves a third of them or more.
-  bool dense(int nc) const {
+  // FP64 hop kernels in the form with three blocks per SM: beyond two waves of two; those of the
+  // iterations for 4D SU(3) below nine waves only where it saves a third of them or more.
+  bool dense() const { return grid.x * grid.y > 2 * 296; }
+  bool dense_iteration(int nc) const {
     const unsigned n = grid.x * grid.y, w2 = (n + 295) / 296, w3 = (n + 443) / 444;
-    if (g.nd == 4 && nc == 3 && w2 < 9) return w2 > 2 && 2 * w2 >= 3 * w3;
-    return w2 > 2;
+    return dense() && (g.nd != 4 || nc != 3 || w2 >= 9 || 2 * w2 >= 3 * w3);
   }
   HopGrid(const EoGeom& geom, int nblk, int tiles, size_t link_bytes) : g(geom), grid(nblk, tiles) {
     if (tiles > 1 && nblk <= 65535 && link_bytes > (size_t)64 << 20) {
@@ -400,7 +400,8 @@ __global__ void __launch_bounds__(128) norm64_kernel(int64_t Vh, EoField f, doub
 // blocks) it is 1.5 % slower.  FP64 solves, usual / dense, by blocks: SU(2) 12^4 648 1.02, 810
 // 1.06, 1296 1.07, 16^4 768 1.06, 2048 1.08; 2D 256^2 768 SU(2) 1.02, SU(3) 1.07, 1536 1.04,
 // 1.11; 3D 32^3 640 1.06, 1.04, 1280 1.14, 1.11.  4D SU(3), waves of two | of three: 3 | 2
-// 1.02 to 1.05, 4 | 3 0.98 to 1.03, 5 | 3 1.01 to 1.06, 6 | 4 1.01, 7 | 5 0.99.  Sloppy kernels keep
+// 1.02 to 1.05, 4 | 3 0.98 to 1.03, 5 | 3 1.01 to 1.06, 6 | 4 1.01, 7 | 5 0.99, but the hop of the
+// updates at four waves 1.04 (8^4, 64 rhs: 25.7 against 26.8 us).  Sloppy kernels keep
 // ptxas's default register target.
 //
 // The kernel bodies below take the block's site block `bx` and rhs tile `by`
@@ -964,7 +965,7 @@ struct Impl {
     const dim3 grid(w.nblk, w.nrhs);
     const HopGrid h = hop_tiles(w);
     const CGState* cst = w.st;
-    if (h.dense(NC)) iterate_hops<DB>(w, st, h, cst, k2);
+    if (h.dense_iteration(NC)) iterate_hops<DB>(w, st, h, cst, k2);
     else iterate_hops<MB>(w, st, h, cst, k2);
     launch(w, st, cg_p_kernel<SP, XP, NCOMP>, grid, dim3(128), w.Vh, w.r, w.p, w.xs, w.st, w.counters);
   }
@@ -990,7 +991,7 @@ struct Impl {
       kernel<<<h.grid, 128, 0, st>>>(h.g, w.hg64, in, par, out, z0, z1, a1, c, w.upd, w.partials, w.counters, res,
                                      w.nblk);
     };
-#define LYM_H64(A, B) run(h.dense(NC) ? hop64_lincomb_kernel<ND, NC, A, B, 3> : hop64_lincomb_kernel<ND, NC, A, B, 1>)
+#define LYM_H64(A, B) run(h.dense() ? hop64_lincomb_kernel<ND, NC, A, B, 3> : hop64_lincomb_kernel<ND, NC, A, B, 1>)
     if (g5in && g5out) LYM_H64(true, true);
     else if (g5in) LYM_H64(true, false);
     else if (g5out) LYM_H64(false, true);
@@ -1034,7 +1035,7 @@ struct Impl {
   static void dslash(Work& w, cudaStream_t st) {
     const HopGrid h = hop_tiles(w);
     w.launches += 1;
-    auto hop = h.dense(NC) ? cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX, DB>
+    auto hop = h.dense() ? cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX, DB>
                          : cg_hop_kernel<ND, NC, SP, GP, COMP, false, R, MX, MB>;
     hop<<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.p, w.s, 1, nullptr);
   }
@@ -1042,9 +1043,9 @@ struct Impl {
     const double k2 = w.kappa * w.kappa;
     const HopGrid h = hop_tiles(w);
     w.launches += 2;
-    auto hop = h.dense(NC) ? cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX, DB>
+    auto hop = h.dense() ? cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX, DB>
                          : cg_hop_kernel<ND, NC, SP, GP, COMP, true, R, MX, MB>;
-    auto rnew = h.dense(NC) ? cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX, DB> : cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX, MB>;
+    auto rnew = h.dense() ? cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX, DB> : cg_rnew_kernel<ND, NC, SP, GP, COMP, R, MX, MB>;
     hop<<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.t, w.s, 1, nullptr);
     rnew<<<h.grid, 128, 0, st>>>(h.g, w.hgs, w.s, w.t, w.r, k2, w.upd,
                                                                       w.partials, w.counters, w.res, w.nblk);
